@@ -92,6 +92,9 @@ int setup_device(int dev)
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return cuda_fail(e, "cudaGetSymbolAddress(allocation-free scratch)");
         g_noalloc_ptr[dev] = static_cast<double*>(p);
+        // so that the allocation-free update's launches take no memory for code either
+        e = preload_update_kernels();
+        if (e != cudaSuccess) return cuda_fail(e, "loading the update's kernels");
     }
     return VD_OK;
 }
@@ -796,7 +799,7 @@ static int plan_update(const vd_box* bx, vd_array4 sborder, const vd_array4 efie
     fill_cfg(a, bx, prm, ns, m.e_id, m.charge[m.e_id]);
     fill_species(a, prm, m);
     int tile[3];
-    transport_tile(dim, tile);
+    transport_tile(dim, prm->precision, tile);
     for (int d = 0; d < 3; d++) {
         const int n = bx->hi[d] - bx->lo[d] + 1;
         a.ntile[d] = (n + tile[d] - 1) / tile[d];

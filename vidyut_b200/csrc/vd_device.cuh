@@ -368,27 +368,28 @@ __device__ __forceinline__ float face_flux_mixed32(const float* u, const float* 
 // Written with the first differences g (of neighbours) and second differences d:
 //   4 beta_1 = 13/3 d_-^2 + (d_- + 2 g_-)^2, 4 beta_2 = 13/3 d_0^2 + (g_- + g_+)^2,
 //   4 beta_3 = 13/3 d_+^2 + (d_+ - 2 g_+)^2
-// and, with q_k = 4 beta_k + 4 eps and tau = 4 |beta_1 - beta_3|, the weights up to a
-// common factor (every weight is a ratio; multiplied through by q_1^2 q_2^2 q_3^2)
-//   WENO-Z   1 + (tau/q_k)^2  ->  Y_k = (q_k^2 + tau^2) prod_(j != k) q_j^2
-//   WENO-JS  1/q_k^2          ->  Y_k = prod_(j != k) q_j^2   (M: then the map)
-// (Source/compute_explicit_flux.H:38-109).  The q_k are first scaled by an exact
-// power of two that brings the larger of q_1, q_3 to [1, 2) (q_2 is at most a few
-// times that), so the products neither overflow nor lose their largest term:
-// densities up to 1e31 leave it above 1e-170.  A reconstruction is then the cell
-// value plus a weighted sum of the candidates' offsets from it, with one reciprocal:
-// where the weights were four divisions per centre and two reconstructions are one
-// each now, the FP64 instructions per face fell from about 250 to about 140, and the
-// 3-D transport of 24 species on 128^3 from 2.85 to @@ ms on B200.
+// and, with q_k = 4 beta_k + 4 eps and tau = |q_1 - q_3|, the weights up to a common
+// factor (every weight is a ratio; multiplied through by q_1^2 q_2^2 q_3^2)
+//   WENO-Z   1 + (tau/q_k)^2  ->  Y_k = P + tau^2 P_k,  P_k = prod_(j != k) q_j^2,  P = q_k^2 P_k
+//   WENO-JS  1/q_k^2          ->  Y_k = P_k   (M: then the map)
+// (Source/compute_explicit_flux.H:38-109).  A reconstruction is then the cell value
+// plus a weighted sum of the candidates' offsets from it, with one reciprocal.  Four
+// divisions per centre and two reconstructions became two reciprocals.
+// Range: the products are of degree 6 in q, so the values are taken scaled by
+// kWenoScale = 2^-32 (exact): eps then keeps q above 2e-39 (q^6 > 1e-232, so a weighted
+// offset keeps its digits down to differences of 1e-60), and values up to 4e32 keep a
+// weighted offset (degree 13) below 1e308.  A larger value overflows to a NaN, and such
+// a face is evaluated again with every centre scaled by its own power of two (SAFE;
+// weno_y64).
 // Every operation is pinned (no contraction left to the compiler), so a centre gives
 // the same bits wherever in a run of faces it is evaluated and the tile
 // decomposition cannot change a result.
+constexpr double kWenoScale = 0x1p-32, kWenoUnscale = 0x1p32;
 
 // 1/d of a normal FP64 number: the hardware's 20-bit approximation and one
 // third-order (Householder) iteration r (1 + e + e^2), e = 1 - d r, which leaves
 // e^3 < 2^-57 beside the rounding; no branch for the special operands that a
-// correctly rounded division serves (d here is a weight sum of order 1e-170 .. 1e3;
-// NaN and infinity give a NaN).
+// correctly rounded division serves (zero, NaN and infinity give a NaN).
 __device__ __forceinline__ double rcp64(double d)
 {
     double r;
@@ -396,34 +397,43 @@ __device__ __forceinline__ double rcp64(double d)
     const double e = __fma_rn(-d, r, 1.0);
     return __fma_rn(r, __fma_rn(e, e, e), r);
 }
+// n/d by the same iteration on the quotient
+__device__ __forceinline__ double div64(double n, double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = __fma_rn(-d, r, 1.0);
+    const double q = __dmul_rn(n, r);
+    return __fma_rn(q, __fma_rn(e, e, e), q);
+}
 struct WenoY64 {
     double y1, y2, y3;
 };
-// S: 1 JS, 2 M (unmapped here), 3 Z; b1..b3 the 4 beta_k
-template <int S>
-__device__ __forceinline__ WenoY64 weno_y64(double b1, double b2, double b3)
+// S: 1 JS, 2 M (unmapped here), 3 Z.  SAFE: the q_k are first scaled by the power of
+// two that brings the larger of q_1, q_3 to [1, 2) (q_2 is at most a few times that;
+// non-negative numbers order like their high words; a NaN or infinity keeps the scale
+// finite and carries itself).
+template <int S, bool SAFE>
+__device__ __forceinline__ WenoY64 weno_y64(double q1, double q2, double q3)
 {
-    constexpr double eps4 = 4e-20;
-    // the exponent field of the larger of q1 and q3 (non-negative numbers order like
-    // their high words); a NaN or infinity keeps the scale finite and carries itself
-    int m = max(max(__double2hiint(b1), __double2hiint(b3)), __double2hiint(eps4));
-    m = min(m, 0x7fd00000) & 0x7ff00000;
-    const double s = __hiloint2double(0x7fe00000 - m, 0);  // 2^-e
-    const double es = __dmul_rn(eps4, s);
-    const double q1 = __fma_rn(b1, s, es), q2 = __fma_rn(b2, s, es), q3 = __fma_rn(b3, s, es);
+    if constexpr (SAFE) {
+        const int m = min(max(__double2hiint(q1), __double2hiint(q3)), 0x7fd00000) & 0x7ff00000;
+        const double s = __hiloint2double(0x7fe00000 - m, 0);  // 2^-e
+        q1 = __dmul_rn(q1, s);
+        q2 = __dmul_rn(q2, s);
+        q3 = __dmul_rn(q3, s);
+    }
     const double Q1 = __dmul_rn(q1, q1), Q2 = __dmul_rn(q2, q2), Q3 = __dmul_rn(q3, q3);
-    const double P1 = __dmul_rn(Q2, Q3), P2 = __dmul_rn(Q1, Q3), P3 = __dmul_rn(Q1, Q2);
     WenoY64 y;
+    y.y1 = __dmul_rn(Q2, Q3);
+    y.y2 = __dmul_rn(Q1, Q3);
+    y.y3 = __dmul_rn(Q1, Q2);
     if constexpr (S == 3) {
-        const double t = __dmul_rn(__dsub_rn(b1, b3), s);
-        const double T = __dmul_rn(t, t);
-        y.y1 = __dmul_rn(__dadd_rn(Q1, T), P1);
-        y.y2 = __dmul_rn(__dadd_rn(Q2, T), P2);
-        y.y3 = __dmul_rn(__dadd_rn(Q3, T), P3);
-    } else {
-        y.y1 = P1;
-        y.y2 = P2;
-        y.y3 = P3;
+        const double t = __dsub_rn(q1, q3);
+        const double T = __dmul_rn(t, t), P = __dmul_rn(Q1, y.y1);
+        y.y1 = __fma_rn(T, y.y1, P);
+        y.y2 = __fma_rn(T, y.y2, P);
+        y.y3 = __fma_rn(T, y.y3, P);
     }
     return y;
 }
@@ -432,7 +442,7 @@ __device__ __forceinline__ double gk_map64(double wk, double g)
 {
     const double num = __fma_rn(wk, wk, __fma_rn(-3.0 * g, wk, g + g * g));
     const double den = __fma_rn(wk, 1.0 - 2.0 * g, g * g);
-    return __dmul_rn(__dmul_rn(wk, num), rcp64(den));
+    return div64(__dmul_rn(wk, num), den);
 }
 // xc + (1/6) sum_k a_k o_k / sum_k a_k with a = (y1, 6 y2, 3 y3) (M: mapped); A2 = 6 y2
 template <int S>
@@ -448,17 +458,23 @@ __device__ __forceinline__ double weno_value64(double xc, double y1, double A2, 
         D = __dadd_rn(__dadd_rn(a1, a2), a3);
     }
     const double N = __fma_rn(a1, o1, __fma_rn(a2, o2, __dmul_rn(a3, o3)));
-    return __fma_rn(1.0 / 6.0, __dmul_rn(N, rcp64(D)), xc);
+    return __fma_rn(1.0 / 6.0, div64(N, D), xc);
 }
 // The sliding window of one field around centre c: value, the differences to its
-// neighbours and the second differences with their 13/3 d^2 terms.
+// neighbours and the second differences d with their 13/3 d^2 + 4 eps.
 struct WenoWin64 {
-    double xc, xp;        // cells c and c + 1
-    double gm, gp;        // x_c - x_(c-1), x_(c+1) - x_c
+    double xc, xp;          // cells c and c + 1
+    double gm, gp;          // x_c - x_(c-1), x_(c+1) - x_c
     double dm, d0, cm, c0;  // second differences at c - 1 and c
 };
-__device__ __forceinline__ double weno_c64(double d) { return __dmul_rn(__dmul_rn(13.0 / 3.0, d), d); }
+template <bool SAFE>
+__device__ __forceinline__ double weno_c64(double d)
+{
+    constexpr double eps4 = SAFE ? 4e-20 : 4e-20 * kWenoScale * kWenoScale;
+    return __fma_rn(__dmul_rn(13.0 / 3.0, d), d, eps4);
+}
 // window around centre c from cells c-2 .. c+1
+template <bool SAFE>
 __device__ __forceinline__ WenoWin64 weno_start64(double xa, double xb, double xc, double xd)
 {
     WenoWin64 w;
@@ -469,29 +485,29 @@ __device__ __forceinline__ WenoWin64 weno_start64(double xa, double xb, double x
     w.gp = __dsub_rn(xd, xc);
     w.dm = __dsub_rn(w.gm, ga);
     w.d0 = __dsub_rn(w.gp, w.gm);
-    w.cm = weno_c64(w.dm);
-    w.c0 = weno_c64(w.d0);
+    w.cm = weno_c64<SAFE>(w.dm);
+    w.c0 = weno_c64<SAFE>(w.d0);
     return w;
 }
 // Both reconstructions around the window's centre, given cell c + 2: `right`, the
 // left-biased value at the right face of c, and `left`, the right-biased value at its
 // left face (each only when wanted); then the window moves on by one cell.
-template <int S, bool RIGHT, bool LEFT>
+template <int S, bool SAFE, bool RIGHT, bool LEFT>
 __device__ __forceinline__ void weno_step64(WenoWin64& w, double xe, double& right, double& left)
 {
-    const double gn = __dsub_rn(xe, w.xp);   // x_(c+2) - x_(c+1)
-    const double dp = __dsub_rn(gn, w.gp);   // second difference at c + 1
-    const double cp = weno_c64(dp);
+    const double gn = __dsub_rn(xe, w.xp);  // x_(c+2) - x_(c+1)
+    const double dp = __dsub_rn(gn, w.gp);  // second difference at c + 1
+    const double cp = weno_c64<SAFE>(dp);
     const double t1 = __fma_rn(2.0, w.gm, w.dm), t2 = __dadd_rn(w.gm, w.gp), t3 = __fma_rn(-2.0, w.gp, dp);
-    const WenoY64 y = weno_y64<S>(__fma_rn(t1, t1, w.cm), __fma_rn(t2, t2, w.c0), __fma_rn(t3, t3, cp));
+    const WenoY64 y = weno_y64<S, SAFE>(__fma_rn(t1, t1, w.cm), __fma_rn(t2, t2, w.c0), __fma_rn(t3, t3, cp));
     const double A2 = __dmul_rn(6.0, y.y2);
     // six times the candidates' offsets from x_c
     if (RIGHT)
-        right = weno_value64<S>(w.xc, y.y1, A2, y.y3, __fma_rn(3.0, w.gm, __dadd_rn(w.dm, w.dm)),
-                                __fma_rn(3.0, w.gp, -w.d0), __fma_rn(3.0, w.gp, -dp));
+        right = weno_value64<S>(w.xc, y.y1, A2, y.y3, __fma_rn(2.0, t1, -w.gm), __fma_rn(3.0, w.gp, -w.d0),
+                                __fma_rn(3.0, w.gp, -dp));
     if (LEFT)
-        left = weno_value64<S>(w.xc, y.y3, A2, y.y1, __fma_rn(-3.0, w.gp, __dadd_rn(dp, dp)),
-                               __fma_rn(-3.0, w.gm, -w.d0), __fma_rn(-3.0, w.gm, -w.dm));
+        left = weno_value64<S>(w.xc, y.y3, A2, y.y1, __fma_rn(2.0, t3, w.gp), __fma_rn(-3.0, w.gm, -w.d0),
+                               __fma_rn(-3.0, w.gm, -w.dm));
     w.xc = w.xp;
     w.xp = xe;
     w.gm = w.gp;
@@ -502,38 +518,36 @@ __device__ __forceinline__ void weno_step64(WenoWin64& w, double xe, double& rig
     w.c0 = cp;
 }
 // local Lax-Friedrichs flux of a face from the reconstructions of the drift flux
-// (fp, fm) and the density (du = up - um) and the two cells' velocities
+// (fp, fm) and the density (up, um) and the two cells' velocities
 // (Source/compute_explicit_flux.H:300-312)
-__device__ __forceinline__ double llf_flux64(double fp, double fm, double du, double vl, double vr)
+__device__ __forceinline__ double llf_flux64(double fp, double fm, double up, double um, double vl, double vr)
 {
     const double lam = fabs(__dmul_rn(0.5, __dadd_rn(vl, vr)));
-    return __dmul_rn(0.5, __fma_rn(lam, du, __dadd_rn(fp, fm)));
+    return __dmul_rn(0.5, __fma_rn(lam, __dsub_rn(up, um), __dadd_rn(fp, fm)));
 }
 
 // ---------------------------------------------------------------------------
 // Face flux from the 6-cell stencil u[0..5] = cells (i-3 .. i+2), velocities v[0..5]
-// (compute_flux, Source/compute_explicit_flux.H:245-316), WENO scheme S.
+// (compute_flux, Source/compute_explicit_flux.H:245-316), WENO scheme S, for values
+// of any size.
 template <int S>
 __device__ __forceinline__ double face_flux_weno64(const double* u, const double* v)
 {
-    double du, fp, fm, r, l;
+    double up, um, fp, fm, x;
     {
-        WenoWin64 w = weno_start64(u[0], u[1], u[2], u[3]);
-        weno_step64<S, true, false>(w, u[4], r, l);
-        double r2;
-        weno_step64<S, false, true>(w, u[5], r2, l);
-        du = __dsub_rn(r, l);
+        WenoWin64 w = weno_start64<true>(u[0], u[1], u[2], u[3]);
+        weno_step64<S, true, true, false>(w, u[4], up, x);
+        weno_step64<S, true, false, true>(w, u[5], x, um);
     }
     {
         double f[6];
 #pragma unroll
         for (int q = 0; q < 6; q++) f[q] = __dmul_rn(u[q], v[q]);
-        WenoWin64 w = weno_start64(f[0], f[1], f[2], f[3]);
-        double d;
-        weno_step64<S, true, false>(w, f[4], fp, d);
-        weno_step64<S, false, true>(w, f[5], d, fm);
+        WenoWin64 w = weno_start64<true>(f[0], f[1], f[2], f[3]);
+        weno_step64<S, true, true, false>(w, f[4], fp, x);
+        weno_step64<S, true, false, true>(w, f[5], x, fm);
     }
-    return llf_flux64(fp, fm, du, v[2], v[3]);
+    return llf_flux64(fp, fm, up, um, v[2], v[3]);
 }
 __device__ __forceinline__ double face_flux_fp64(const double* u, const double* v, int hyp_order, int scheme,
                                                  double dxmin, double dt)
@@ -542,6 +556,17 @@ __device__ __forceinline__ double face_flux_fp64(const double* u, const double* 
     if (scheme == 3) return face_flux_weno64<3>(u, v);
     if (scheme == 2) return face_flux_weno64<2>(u, v);
     return face_flux_weno64<1>(u, v);
+}
+// The face of a run whose scaled evaluation was not finite: from its staged (scaled)
+// densities pu and velocity basis pb (null: velocity k), `str` apart; scaled result.
+static __device__ __noinline__ double face_flux_again64(const double* pu, const double* pb, int str, double k, int scheme)
+{
+    double u[6], v[6];
+    for (int q = 0; q < 6; q++) {
+        u[q] = pu[q * str] * kWenoUnscale;
+        v[q] = pb ? __dmul_rn(k, pb[q * str]) : k;
+    }
+    return face_flux_fp64(u, v, 5, scheme, 1.0, 0.0) * kWenoScale;
 }
 
 // ---------------------------------------------------------------------------

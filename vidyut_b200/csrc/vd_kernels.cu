@@ -644,17 +644,25 @@ void finish_species_lists(TransportArgs& a, const VdMechDev& m)
     }
 }
 
-void transport_tile(int dim, int t[3])
+template <class TS>
+static void tile_of(int t[3])
 {
-    if (dim == 1) { t[0] = DefaultTile<1>::T::X; t[1] = 1; t[2] = 1; }
-    else if (dim == 2) { t[0] = DefaultTile<2>::T::X; t[1] = DefaultTile<2>::T::Y; t[2] = 1; }
-    else { t[0] = DefaultTile<3>::T::X; t[1] = DefaultTile<3>::T::Y; t[2] = DefaultTile<3>::T::Z; }
+    t[0] = TS::X;
+    t[1] = TS::Y;
+    t[2] = TS::Z;
+}
+void transport_tile(int dim, int prec, int t[3])
+{
+    if (dim == 1) tile_of<DefaultTile<1, PREC_FP64>::T>(t);
+    else if (dim == 2) tile_of<DefaultTile<2, PREC_FP64>::T>(t);
+    else if (prec == PREC_MIXED) tile_of<DefaultTile<3, PREC_MIXED>::T>(t);
+    else tile_of<DefaultTile<3, PREC_FP64>::T>(t);
 }
 
 template <int DIM, int PREC, int MINB>
 static cudaError_t launch_tr(const TransportArgs& a, cudaStream_t st)
 {
-    using TS = typename DefaultTile<DIM>::T;
+    using TS = typename DefaultTile<DIM, PREC>::T;
     constexpr int GRP = group_fit<DIM, PREC, TS, MINB>();
     const size_t smem = transport_smem<DIM, PREC, TS, GRP>(a.nb);
     static unsigned attr_set = 0;  // one bit per device
@@ -668,7 +676,7 @@ static cudaError_t launch_tr(const TransportArgs& a, cudaStream_t st)
     }
     unsigned nt = (unsigned)a.ntile[0] * a.ntile[1] * a.ntile[2];
     ProfScope ps("k_transport", st);
-    k_transport<DIM, PREC, MINB><<<nt, DefaultTile<DIM>::T::NTH, smem, st>>>(a);
+    k_transport<DIM, PREC, MINB><<<nt, TS::NTH, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -766,6 +774,34 @@ cudaError_t launch_joule_pre(const TransportArgs& a, int dim, int prec, cudaStre
     if (dim == 1) return launch_jp<1, PREC_FP64>(a, st);
     if (dim == 2) return launch_jp<2, PREC_FP64>(a, st);
     return launch_jp<3, PREC_FP64>(a, st);
+}
+
+// Loads the code of the kernels an update launches (modules load lazily: a kernel's
+// first launch may take device memory for it otherwise).
+template <int DIM, int PREC>
+static cudaError_t load_update_kernels()
+{
+    cudaFuncAttributes fa;
+    const int mb = g_tr_minb[DIM][PREC];
+    const void* fn = (const void*)k_transport<DIM, PREC, 1>;
+    if (mb == 2) fn = (const void*)k_transport<DIM, PREC, 2>;
+    if constexpr (DIM < 3) {
+        if (mb == 3) fn = (const void*)k_transport<DIM, PREC, 3>;
+        if (mb == 4) fn = (const void*)k_transport<DIM, PREC, 4>;
+    }
+    cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)k_joule_pre<DIM, PREC>);
+    return e;
+}
+cudaError_t preload_update_kernels()
+{
+    cudaError_t e = load_update_kernels<1, PREC_FP64>();
+    if (e == cudaSuccess) e = load_update_kernels<2, PREC_FP64>();
+    if (e == cudaSuccess) e = load_update_kernels<3, PREC_FP64>();
+    if (e == cudaSuccess) e = load_update_kernels<1, PREC_MIXED>();
+    if (e == cudaSuccess) e = load_update_kernels<2, PREC_MIXED>();
+    if (e == cudaSuccess) e = load_update_kernels<3, PREC_MIXED>();
+    return e;
 }
 
 cudaError_t launch_transport(const TransportArgs& a, int dim, int prec, cudaStream_t st)

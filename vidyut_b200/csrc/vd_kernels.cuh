@@ -154,12 +154,13 @@ cudaError_t launch_prep(const PrepArgs& a, int prec, int ns, cudaStream_t st);
 // launch_transport.
 cudaError_t launch_joule_pre(const TransportArgs& a, int dim, int prec, cudaStream_t st);
 cudaError_t launch_transport(const TransportArgs& a, int dim, int prec, cudaStream_t st);
+cudaError_t preload_update_kernels();
 cudaError_t launch_checksums(const BoxIdx& b, const A4& rxn, const A4& pn, double* out, cudaStream_t st);
 cudaError_t launch_time_scales(const BoxIdx& b, int dim, const A4& st, const TransportArgs& a,
                                unsigned long long* out, cudaStream_t s);
 
 // Tile shape used by the transport kernel for a given dimension (for host-side tiling).
-void transport_tile(int dim, int tile[3]);
+void transport_tile(int dim, int prec, int tile[3]);
 
 // Launch accounting: every launch increments a counter; when profiling is on it is
 // bracketed by CUDA events on its stream (see vd_profile_* in the header).

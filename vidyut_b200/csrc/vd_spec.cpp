@@ -391,6 +391,11 @@ int spec_build(const VdMechDev& m)
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->batch[PREC_FP64], mod->lib, "vd_spec_prep_batch_fp64");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->batch[PREC_MIXED], mod->lib, "vd_spec_prep_batch_mixed");
     if (e == cudaSuccess) {
+        // load the code now, not at the first launch
+        cudaFuncAttributes fa;
+        for (int p = 0; p < 2 && e == cudaSuccess; p++) e = cudaFuncGetAttributes(&fa, (const void*)mod->prep[p]);
+    }
+    if (e == cudaSuccess) {
         // layout check of the kernel argument struct
         cudaKernel_t sz;
         unsigned long long* d = nullptr;

@@ -87,11 +87,16 @@ template <int X_, int Y_, int Z_, int NTH_>
 struct TileShape {
     static constexpr int X = X_, Y = Y_, Z = Z_, NTH = NTH_;
 };
-template <int DIM> struct DefaultTile;
-template <> struct DefaultTile<1> { using T = TileShape<256, 1, 1, 256>; };
-template <> struct DefaultTile<2> { using T = TileShape<32, 8, 1, 256>; };
-template <> struct DefaultTile<3> { using T = TileShape<8, 8, 8, 512>; };
-template <int DIM> constexpr int default_nth() { return DIM == 3 ? 512 : 256; }
+// Tile of the per-box kernel.  In 3-D FP64 the 384 runs of faces per species make one
+// pass of 384 threads at 80 registers: with 512 threads at 64 registers the face loop
+// spills (1.67 against 1.61 ms for 24 species on 128^3; 16x4x4 tiles of 192 threads,
+// four per SM, 1.68 ms).
+template <int DIM, int PREC> struct DefaultTile;
+template <int PREC> struct DefaultTile<1, PREC> { using T = TileShape<256, 1, 1, 256>; };
+template <int PREC> struct DefaultTile<2, PREC> { using T = TileShape<32, 8, 1, 256>; };
+template <> struct DefaultTile<3, PREC_FP64> { using T = TileShape<8, 8, 8, 384>; };
+template <> struct DefaultTile<3, PREC_MIXED> { using T = TileShape<8, 8, 8, 512>; };
+template <int DIM, int PREC> constexpr int default_nth() { return DefaultTile<DIM, PREC>::T::NTH; }
 
 template <int DIM, class TS>
 struct TileGeom {
@@ -116,7 +121,7 @@ struct RunGeom {
     }
     static constexpr int R0 = NL(0) * NR(0), R1 = NL(1) * NR(1), R2 = NL(2) * NR(2);
     static constexpr int ROFF1 = R0, ROFF2 = R0 + R1, NRUN = R0 + R1 + R2;
-    static_assert(RUN >= 1 && RUN <= 60, "run length fits the info fields");
+    static_assert(RUN >= 1 && RUN <= 30, "run length fits the info fields");
 };
 
 template <int PREC> struct VelT { using T = double; };
@@ -385,60 +390,92 @@ __device__ __forceinline__ bool staged_cell(const TransportArgs& a, int cc, cons
     return ok;
 }
 
-// velocity bases of staged position cc of direction D: sB[k*STOT + cc] for slot k;
-// so[cc]: the position's cell offset in the state (-1: stages as zero), read by
-// every species group's staging
-template <int DIM, int PREC, int D, class TS>
-__device__ __forceinline__ bool stage_basis(const TransportArgs& a, int cc, const int* org,
-                                            typename VelT<PREC>::T* sB, JStage js, bool jst, int* so)
+// What the velocity bases of one staged position are made from, loaded ahead of the
+// arithmetic so that several positions' loads are in flight together.
+struct BasisIn {
+    int D;           // sweep direction of the position's line set
+    int o;           // cell offset in the state, -1: stages as zero (see soffs)
+    int64_t off;     // the same in 64 bits (valid when ok)
+    bool ok;
+    double E, N, Te, ne, emag;
+};
+// staged position c of the tile (line sets of all directions in one index range)
+template <int DIM, int PREC, class TS>
+__device__ __forceinline__ BasisIn basis_load(const TransportArgs& a, int c, const int* org, bool jst)
 {
-    bool bad = false;  // a NaN or infinity in the position's E, Te or density sum
     using G = TileGeom<DIM, TS>;
-    using VT = typename VelT<PREC>::T;
+    BasisIn w;
     int g[3];
-    const bool ok = staged_cell<DIM, D, TS>(a, cc, org, g);
-    VT b[3] = {VT(0), VT(0), VT(0)};
-    double ne = 0.0, Te = 0.0, N = 0.0;
-    so[cc] = ok ? (int)a.sb.off(g[0], g[1], g[2]) : -1;
-    if (ok) {
+    w.D = 0;
+    if (DIM > 2 && c >= G::SOFF2) {
+        w.D = 2;
+        w.ok = staged_cell<DIM, (DIM > 2 ? 2 : 0), TS>(a, c - G::SOFF2, org, g);
+    } else if (DIM > 1 && c >= G::SOFF1) {
+        w.D = 1;
+        w.ok = staged_cell<DIM, (DIM > 1 ? 1 : 0), TS>(a, c - G::SOFF1, org, g);
+    } else {
+        w.ok = staged_cell<DIM, 0, TS>(a, c, org, g);
+    }
+    w.ok = w.ok && c < G::STOT;
+    w.off = 0;
+    w.o = -1;
+    w.E = w.N = w.Te = w.ne = w.emag = 0.0;
+    if (w.ok) {
         const int ns = a.ns;
         const int64_t cs = a.sb.ns;
-        const double* p = a.sb.p + a.sb.off(g[0], g[1], g[2]);
-        const double E = p[(VD_EFX(ns) + D) * cs];
-        N = a.Nv(g[0], g[1], g[2]);
-        Te = p[VD_ETEMP(ns) * cs];
-        bad = !(isfinite(E) && isfinite(Te) && isfinite(N));
-        if (joule_staged<DIM, PREC>() && jst) ne = p[a.e_id * cs];
+        w.off = a.sb.off(g[0], g[1], g[2]);
+        w.o = (int)w.off;
+        const double* p = a.sb.p + w.off;
+        w.E = __ldg(p + (VD_EFX(ns) + w.D) * cs);
+        w.N = a.Nv(g[0], g[1], g[2]);
+        w.Te = __ldg(p + VD_ETEMP(ns) * cs);
+        if (joule_staged<DIM, PREC>() && jst) w.ne = __ldg(p + a.e_id * cs);
         // |E| of the three state components, as compute_vel takes it
         // (Source/PlasmaChem.H:194-196), for the models in |E| and |E|/N
-        double emag = 0.0;
         if (a.stage_emag) {
             const double ex = p[VD_EFX(ns) * cs], ey = p[VD_EFY(ns) * cs], ez = p[VD_EFZ(ns) * cs];
-            emag = sqrt(ex * ex + ey * ey + ez * ez);
+            w.emag = sqrt(ex * ex + ey * ey + ez * ez);
         }
-        for (int k = 0; k < a.nb; k++) {
+    }
+    return w;
+}
+// velocity bases of staged position c: sB[k*STOT + c] for slot k; so[c]: its cell
+// offset in the state, read by every species group's staging; returns whether its E,
+// Te or density sum is a NaN or infinity
+template <int DIM, int PREC, class TS>
+__device__ __forceinline__ bool basis_store(const TransportArgs& a, int c, const BasisIn& w,
+                                            typename VelT<PREC>::T* sB, JStage js, bool jst, int* so)
+{
+    using G = TileGeom<DIM, TS>;
+    using VT = typename VelT<PREC>::T;
+    so[c] = w.o;
+#pragma unroll
+    for (int k = 0; k < kMaxBases; k++) {
+        if (k >= a.nb) break;
+        VT b = VT(0);
+        if (w.ok) {
             const int kind = a.bkind[k];
             if constexpr (PREC == PREC_FP64) {
-                if (kind == 0) b[k] = E / (sqrt(Te) * N);
-                else if (kind == 1) b[k] = E / N;
-                else if (kind == 2) b[k] = E;
-                else b[k] = basis_field_fp64(kind, a.bfit[k], a.bpow[k], E, emag, N, Te);
+                if (kind == 0) b = w.E * rsqrt(w.Te) * rcp64(w.N);
+                else if (kind == 1) b = w.E * rcp64(w.N);
+                else if (kind == 2) b = w.E;
+                else b = basis_field_fp64(kind, a.bfit[k], a.bpow[k], w.E, w.emag, w.N, w.Te);
             } else {
-                const float Ef = (float)E, rN = rcp_approx((float)N);
-                if (kind == 0) b[k] = Ef * rsqrtf((float)Te) * rN;
-                else if (kind == 1) b[k] = Ef * rN;
-                else if (kind == 2) b[k] = Ef;
-                else b[k] = basis_field_f32(kind, a.bfit[k], (float)a.bpow[k], Ef, (float)emag, (float)N, (float)Te);
+                const float Ef = (float)w.E, rN = rcp_approx((float)w.N);
+                if (kind == 0) b = Ef * rsqrtf((float)w.Te) * rN;
+                else if (kind == 1) b = Ef * rN;
+                else if (kind == 2) b = Ef;
+                else b = basis_field_f32(kind, a.bfit[k], (float)a.bpow[k], Ef, (float)w.emag, (float)w.N, (float)w.Te);
             }
         }
+        sB[k * G::STOT + c] = b;
     }
-    for (int k = 0; k < a.nb; k++) sB[k * G::STOT + cc] = b[k];
     if (joule_staged<DIM, PREC>() && jst) {
-        js.ne[cc] = ne;
-        js.te[cc] = (float)Te;
-        js.nd[cc] = (float)N;
+        js.ne[c] = w.ne;
+        js.te[c] = (float)w.Te;
+        js.nd[c] = (float)w.N;
     }
-    return bad;
+    return w.ok && !(isfinite(w.E) && isfinite(w.Te) && isfinite(w.N));
 }
 
 // density of species s at staged position cc of direction D
@@ -614,10 +651,12 @@ __device__ __forceinline__ void run_faces(const TransportArgs& a, int2 ri, int z
     const VT* const pb = sB ? sB + base : nullptr;
     auto den = [&](int i) -> double { return (double)pu[i * STR]; };
     auto vel = [&](int i) -> double { return pb ? __dmul_rn(k, pb[i * STR]) : (double)k; };
-    auto store = [&](int i, VT F) {
-        if (i >= nok || (i == ilo && zlo) || (i == ihi && zhi)) F = VT(0);
-        sF[fbase + i * STR] = F;
-    };
+    // faces stored as zero: beyond the box, and IHNEUBC domain faces
+    unsigned long long zero = ~0ull << nok;
+    if (zlo && ilo >= 0) zero |= 1ull << ilo;
+    if (zhi && ihi >= 0) zero |= 1ull << ihi;
+    VT* const pf = sF + fbase;
+    auto store = [&](int i, VT F) { pf[i * STR] = (zero >> i) & 1 ? VT(0) : F; };
     if constexpr (S == 0) {
         // upwind / WAF: the window of densities and velocities slides along the run
         double um = den(1), uL = den(2), uR = den(3), vL = vel(2);
@@ -633,42 +672,60 @@ __device__ __forceinline__ void run_faces(const TransportArgs& a, int2 ri, int z
         }
     } else {
         // One field at a time (the densities u, then the drift fluxes f = u v), so that
-        // only one field's window is live; face i lies between centres i + 2 (left)
-        // and i + 3 (right), whose reconstructions follow each other.  The densities'
-        // up - um waits in the face's flux slot, and the loops stay rolled: no
-        // per-face register arrays and little code.
+        // only one field's window is live (both at once need 128 registers: 2.24 ms
+        // for the 3-D transport of 24 species on 128^3 against 1.61 ms); face i lies
+        // between centres i + 2 (left) and i + 3 (right), whose reconstructions follow
+        // each other.  The densities' up - um waits in the face's flux slot.  Unrolled by
+        // two, the windows need no register moves; unrolled over the whole run the code
+        // overflows the instruction cache (2.54 against 1.92 ms then).
         static_assert(PREC == PREC_FP64, "runs of faces serve the FP64 path");
+        int big = 0;  // the largest high word of |F|
         {
-            WenoWin64 w = weno_start64(den(0), den(1), den(2), den(3));
+            WenoWin64 w = weno_start64<false>(den(0), den(1), den(2), den(3));
             double r, l, rn;
-            weno_step64<S, true, false>(w, den(4), r, l);
+            weno_step64<S, false, true, false>(w, den(4), r, l);
             const VT* pe = pu + 5 * STR;
-            VT* pf = sF + fbase;
-#pragma unroll 1
+            VT* pd = pf;
+#pragma unroll 2
             for (int i = 0; i < nf; i++) {
-                weno_step64<S, true, true>(w, *pe, rn, l);
-                *pf = __dsub_rn(r, l);
+                weno_step64<S, false, true, true>(w, *pe, rn, l);
+                *pd = __dsub_rn(r, l);
                 r = rn;
                 pe += STR;
-                pf += STR;
+                pd += STR;
             }
         }
         {
-            auto flx = [&](int i) -> double { return __dmul_rn(den(i), vel(i)); };
             double vl = vel(2), vr = vel(3), v1 = vel(4);
-            WenoWin64 w = weno_start64(flx(0), flx(1), __dmul_rn(den(2), vl), __dmul_rn(den(3), vr));
+            WenoWin64 w = weno_start64<false>(__dmul_rn(den(0), vel(0)), __dmul_rn(den(1), vel(1)),
+                                              __dmul_rn(den(2), vl), __dmul_rn(den(3), vr));
             double r, l, rn;
-            weno_step64<S, true, false>(w, __dmul_rn(den(4), v1), r, l);
-#pragma unroll 1
+            weno_step64<S, false, true, false>(w, __dmul_rn(den(4), v1), r, l);
+            const VT* pe = pu + 5 * STR;
+            const VT* pb5 = pb + 5 * STR;
+            VT* pd = pf;
+            unsigned z = (unsigned)zero;
+#pragma unroll 2
             for (int i = 0; i < nf; i++) {
-                const double v2 = vel(i + 5);
-                weno_step64<S, true, true>(w, __dmul_rn(den(i + 5), v2), rn, l);
-                store(i, (VT)llf_flux64(r, l, sF[fbase + i * STR], vl, vr));
+                const double v2 = pb ? __dmul_rn(k, *pb5) : (double)k;
+                weno_step64<S, false, true, true>(w, __dmul_rn(*pe, v2), rn, l);
+                const double F = llf_flux64(r, l, *pd, 0.0, vl, vr);
+                big = max(big, __double2hiint(F) & 0x7fffffff);
+                *pd = z & 1 ? 0.0 : F;
+                z >>= 1;
                 r = rn;
                 vl = vr;
                 vr = v1;
                 v1 = v2;
+                pe += STR;
+                pb5 += STR;
+                pd += STR;
             }
+        }
+        const bool again = big >= 0x7ff00000;
+        if (again) {
+#pragma unroll 1
+            for (int i = 0; i < nf; i++) store(i, face_flux_again64(pu + i * STR, pb ? pb + i * STR : nullptr, STR, k, S));
         }
     }
 }
@@ -693,6 +750,9 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
     using SM = TileSmem<DIM, PREC, TS>;
     constexpr int RUN = run_len<DIM, TS>();
     using RG = RunGeom<DIM, TS, RUN>;
+    // FP64 WENO takes its densities scaled (kWenoScale, exact), and so its fluxes
+    const bool scaled = PREC == PREC_FP64 && a.hyp_order == 5;
+    const double usc = scaled ? kWenoScale : 1.0, uisc = scaled ? kWenoUnscale : 1.0;
     double* sJ = reinterpret_cast<double*>(smem);  // mixed path only
     int2* sRI = reinterpret_cast<int2*>(smem + SM::joule());  // by_runs
     int* sFI = reinterpret_cast<int*>(smem + SM::joule());    // single faces
@@ -709,21 +769,52 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
     const JStage js{reinterpret_cast<double*>(dens), reinterpret_cast<float*>(dens + G::STOT * sizeof(double)),
                     reinterpret_cast<float*>(dens + G::STOT * (sizeof(double) + sizeof(float)))};
 
-    // own cell
-    const int cx = tid % G::T[0], cy = (tid / G::T[0]) % G::T[1], cz = tid / (G::T[0] * G::T[1]);
-    const int gi = org[0] + cx, gj = org[1] + cy, gk = org[2] + cz;
-    const bool own = (tid < G::NCELL) && gi <= a.hi[0] && gj <= a.hi[1] && gk <= a.hi[2];
     const int ns = a.ns;
     const int64_t cs = a.sb.ns;
-    const int64_t own_o = own ? a.sb.off(gi, gj, gk) : 0;
+    bool bad = false;  // this thread met a NaN or infinity (reported once per warp at the end)
+    // The own cells of a thread: cell tid of the tile, and every NTH-th after it
+    // where the CTA has fewer threads than the tile has cells.
+    struct Own {
+        int cx, cy, cz, gi, gj, gk;
+        int64_t o, r, p;  // offsets in the state, the reaction source and the output
+        bool ok;       // inside the box
+        double ne_new, een_new;
+    };
+    constexpr bool kOne = NTH >= G::NCELL;  // one own cell per thread
+    auto own_cell = [&](int c) {
+        Own w;
+        w.cx = c % TS::X;
+        w.cy = (c / TS::X) % TS::Y;
+        w.cz = c / (TS::X * TS::Y);
+        w.gi = org[0] + w.cx;
+        w.gj = org[1] + w.cy;
+        w.gk = org[2] + w.cz;
+        w.ok = c < G::NCELL && w.gi <= a.hi[0] && w.gj <= a.hi[1] && w.gk <= a.hi[2];
+        w.o = w.ok ? a.sb.off(w.gi, w.gj, w.gk) : 0;
+        w.r = w.ok ? a.rxn.off(w.gi, w.gj, w.gk) : 0;
+        w.p = w.ok ? a.pn.off(w.gi, w.gj, w.gk) : 0;
+        w.ne_new = w.een_new = 0.0;
+        return w;
+    };
+    Own own1;
+    if constexpr (kOne) own1 = own_cell(tid);
+    auto each_own = [&](auto&& fn) {
+        if constexpr (kOne) {
+            if (own1.ok) fn(own1);
+        } else {
+#pragma unroll 1
+            for (int c = tid; c < G::NCELL; c += NTH) {
+                Own w = own_cell(c);
+                if (w.ok) fn(w);
+            }
+        }
+    };
     // The own cell's state and reaction source are read-only in this kernel (the
     // update goes to a.pn): read through the non-coherent path, so that these
     // loads may be issued ahead of the cell's stores.
-    const int64_t own_r = own ? a.rxn.off(gi, gj, gk) : 0;
-    auto state = [&](int s) -> double { return __ldg(a.sb.p + own_o + s * cs); };
-    auto rate = [&](int s) -> double { return __ldg(a.rxn.p + own_r + s * a.rxn.ns); };
-    double ne_new = 0.0, een_new = 0.0;
-    bool bad = false;  // this thread met a NaN or infinity (reported once per warp at the end)
+    auto state = [&](const Own& w, int s) -> double { return __ldg(a.sb.p + w.o + s * cs); };
+    auto out = [&](const Own& w, int s) -> double& { return a.pn.p[w.p + s * a.pn.ns]; };
+    auto rate = [&](const Own& w, int s) -> double { return __ldg(a.rxn.p + w.r + s * a.rxn.ns); };
     const int nfl = a.nfl;
     // the mixed path's Joule faces, evaluated here (a barrier follows them)
     const bool jin = joule_in_tile(a, PREC);
@@ -731,8 +822,8 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
     // Joule term of the own cell from the tile's faces: half the sum of its faces,
     // each domain face replaced as the reference does
     // (Source/ElecEnergySource.cpp:84-94,153-162)
-    auto joule_own = [&]() -> double {
-        const int gc[3] = {gi, gj, gk}, lc[3] = {cx, cy, cz};
+    auto joule_own = [&](const Own& w) -> double {
+        const int gc[3] = {w.gi, w.gj, w.gk}, lc[3] = {w.cx, w.cy, w.cz};
         double jheat = 0.0;
 #pragma unroll
         for (int d = 0; d < DIM; d++) {
@@ -754,19 +845,19 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
     };
 
     // one species' own-cell result
-    // (st: the species' old value, state(s), loaded by the caller so that several
+    // (st: the species' old value, state(w, s), loaded by the caller so that several
     // species' loads can be in flight together)
-    auto finish = [&](int s, double acc, double st) {
+    auto finish = [&](Own& w, int s, double acc, double st) {
         if (s == ns) {
             if (jin) {
-                const double jh = joule_own();
+                const double jh = joule_own(w);
                 acc += jh;
-                a.pn(gi, gj, gk, VD_EJH(ns)) = jh;
+                out(w, VD_EJH(ns)) = jh;
             } else {
                 // the Joule term the joule_tile pass left in EJH
-                acc += a.pn(gi, gj, gk, VD_EJH(ns));
+                acc += out(w, VD_EJH(ns));
             }
-            if (a.write_diag) a.pn(gi, gj, gk, VD_EIH(ns)) = rate(ns);
+            if (a.write_diag) out(w, VD_EIH(ns)) = rate(w, ns);
         }
         double nn = st + a.dt * acc;
         if (a.bound_specden && s != ns) {
@@ -775,10 +866,10 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
             if (nn < lo) nn = lo;
         }
         bad |= !isfinite(nn);
-        a.pn(gi, gj, gk, s) = nn;
-        if (a.dsdt.p) a.dsdt(gi, gj, gk, s) = acc;
-        if (s == a.e_id) ne_new = nn;
-        if (s == ns) een_new = nn;
+        out(w, s) = nn;
+        if (a.dsdt.p) a.dsdt(w.gi, w.gj, w.gk, s) = acc;
+        if (s == a.e_id) w.ne_new = nn;
+        if (s == ns) w.een_new = nn;
     };
 
     if (nfl > 0) {
@@ -788,36 +879,19 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
         } else {
             for (int f = tid; f < G::FTOT; f += NTH) sFI[f] = face_info<DIM, TS>(a, f, org);
         }
-        if constexpr (PREC == PREC_MIXED) {
-            // one loop per direction's line set, two positions per iteration, so
-            // that the loads of both positions are in flight together (measured
-            // faster for the mixed tile, slower for the FP64 one, whose positions
-            // then split less evenly over the threads)
-            auto bases = [&](auto dtag) {
-                constexpr int D = decltype(dtag)::value;
-                constexpr int off = D == 0 ? 0 : (D == 1 ? G::SOFF1 : G::SOFF2);
-                const JStage jd{js.ne + off, js.te + off, js.nd + off};
-#pragma unroll 2
-                for (int cc = tid; cc < G::template NS<D>(); cc += NTH)
-                    bad |= stage_basis<DIM, PREC, D, TS>(a, cc, org, sB + off, jd, jin, sSO + off);
-            };
-            bases(std::integral_constant<int, 0>{});
-            if constexpr (DIM > 1) bases(std::integral_constant<int, 1>{});
-            if constexpr (DIM > 2) bases(std::integral_constant<int, 2>{});
-        } else {
-            for (int c = tid; c < G::STOT; c += NTH) {
-                if (c < G::SOFF1) {
-                    bad |= stage_basis<DIM, PREC, 0, TS>(a, c, org, sB, js, jin, sSO);
-                } else if (DIM > 1 && c < G::SOFF2) {
-                    const JStage j1{js.ne + G::SOFF1, js.te + G::SOFF1, js.nd + G::SOFF1};
-                    bad |= stage_basis<DIM, PREC, (DIM > 1 ? 1 : 0), TS>(a, c - G::SOFF1, org, sB + G::SOFF1, j1,
-                                                                         jin, sSO + G::SOFF1);
-                } else if (DIM > 2) {
-                    const JStage j2{js.ne + G::SOFF2, js.te + G::SOFF2, js.nd + G::SOFF2};
-                    bad |= stage_basis<DIM, PREC, (DIM > 2 ? 2 : 0), TS>(a, c - G::SOFF2, org, sB + G::SOFF2, j2,
-                                                                         jin, sSO + G::SOFF2);
-                }
-            }
+        // PB positions per thread at a time, their loads in flight together: two for
+        // FP64 (1.61 ms; 4 take 1.63 ms and 7 as much), one for the mixed path, where
+        // the smaller loop counts for more (3-D 1.86 ms, 3 at a time 1.87 ms; 2-D 80.3
+        // and 84.2 us)
+        constexpr int PB = PREC == PREC_FP64 ? 2 : 1;
+#pragma unroll 1
+        for (int c0 = tid; c0 < G::STOT; c0 += PB * NTH) {
+            BasisIn w[PB];
+#pragma unroll
+            for (int k = 0; k < PB; k++) w[k] = basis_load<DIM, PREC, TS>(a, c0 + k * NTH, org, jin);
+#pragma unroll
+            for (int k = 0; k < PB; k++)
+                if (c0 + k * NTH < G::STOT) bad |= basis_store<DIM, PREC, TS>(a, c0 + k * NTH, w[k], sB, js, jin, sSO);
         }
         // the offset table and the staged Joule inputs are read by other threads
         if (stab || (joule_staged<DIM, PREC>() && jin)) __syncthreads();
@@ -872,30 +946,36 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
             if constexpr (joule_staged<DIM, PREC>()) __syncthreads();
         }
     }
-    for (int g0 = 0; g0 < nfl; g0 += GRP) {
-        const int gn = nfl - g0 < GRP ? nfl - g0 : GRP;
-        // (1) densities of the group on the staged lines
-        if (stab) {
-            // four positions per thread at a time: their loads in flight together
-            constexpr int CH = 4;
-            const int tot = gn * G::STOT;
-            for (int q0 = tid; q0 < tot; q0 += CH * NTH) {
-                VT u[CH];
+    // (1) densities of a species group on the staged lines.  Element tid + k NTH of the
+    // group's gn x STOT staged values, k = 0 .. PF-1, is fetched into registers
+    // (stage_fetch) before the barrier that ends the previous group's faces and
+    // written behind that group's divergence (stage_put), so that the loads' latency
+    // passes while the CTA waits and updates its cells; the rest of a large group
+    // follows in chunks of CH loads.  Four ahead for the mixed path (3-D 1.86 ms; one
+    // 1.96, eight 1.87 ms), one for FP64, whose registers are short (1.61 ms; eight
+    // 1.66 ms); chunks of 8 (of 4: FP64 1.73 ms).
+    constexpr int PFX = PREC == PREC_FP64 ? 1 : 4;
+    constexpr int PF = (GRP * G::STOT + NTH - 1) / NTH < PFX ? (GRP * G::STOT + NTH - 1) / NTH : PFX;
+    constexpr int CH = 8;
+    auto stage_load = [&](int g0, int gn, int q) -> double {
+        if (q >= gn * G::STOT) return 0.0;
+        const int j = GRP == 1 ? 0 : q / G::STOT, o = sSO[q - j * G::STOT];
+        return o >= 0 ? __ldg(a.sb.p + o + (int64_t)a.fl_sp[g0 + j] * cs) : 0.0;
+    };
+    auto stage_store = [&](int gn, int q, double v) {
+        if (q < gn * G::STOT) sU[q] = (VT)(PREC == PREC_FP64 ? v * usc : v);
+    };
+    auto stage_rest = [&](int g0, int gn, int k0) {
+        for (int q0 = tid + k0 * NTH; q0 < gn * G::STOT; q0 += CH * NTH) {
+            double v[CH];
 #pragma unroll
-                for (int k = 0; k < CH; k++) {
-                    const int q = q0 + k * NTH;
-                    u[k] = VT(0);
-                    if (q < tot) {
-                        const int j = q / G::STOT, c = q - j * G::STOT;
-                        const int o = sSO[c];
-                        if (o >= 0) u[k] = (VT)__ldg(a.sb.p + o + (int64_t)a.fl_sp[g0 + j] * cs);
-                    }
-                }
+            for (int k = 0; k < CH; k++) v[k] = stage_load(g0, gn, q0 + k * NTH);
 #pragma unroll
-                for (int k = 0; k < CH; k++)
-                    if (q0 + k * NTH < tot) sU[q0 + k * NTH] = u[k];
-            }
-        } else for (int q = tid; q < gn * G::STOT; q += NTH) {
+            for (int k = 0; k < CH; k++) stage_store(gn, q0 + k * NTH, v[k]);
+        }
+    };
+    auto stage_far = [&](int g0, int gn) {  // offsets beyond 32 bits: no table
+        for (int q = tid; q < gn * G::STOT; q += NTH) {
             const int j = q / G::STOT, c = q - j * G::STOT;
             const int s = a.fl_sp[g0 + j];
             VT u;
@@ -906,16 +986,25 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
             } else {
                 u = stage_density<DIM, PREC, (DIM > 2 ? 2 : 0), TS>(a, c - G::SOFF2, s, org);
             }
+            if constexpr (PREC == PREC_FP64) u *= usc;
             sU[q] = u;
         }
+    };
+    if (nfl > 0) {
+        const int gn = nfl < GRP ? nfl : GRP;
+        if (stab) stage_rest(0, gn, 0);
+        else stage_far(0, gn);
         __syncthreads();
+    }
+    for (int g0 = 0; g0 < nfl; g0 += GRP) {
+        const int gn = nfl - g0 < GRP ? nfl - g0 : GRP;
         // (2) every face flux of the group: by runs of faces along the lines, or
         // face by face
         // face by face; one loop per scheme family, so that the WENO loop carries
         // no low-order code
         auto runs = [&](auto sch) {
             for (int q = tid; q < gn * RG::NRUN; q += NTH) {
-                const int j = q / RG::NRUN, r = q - j * RG::NRUN;
+const int j = GRP == 1 ? 0 : q / RG::NRUN, r = q - j * RG::NRUN;
                 const int sl = a.fl_slot[g0 + j];
                 run_faces<DIM, PREC, TS, RUN, decltype(sch)::value>(a, sRI[r], a.fl_zm[g0 + j], sU + j * G::STOT,
                                                                    sl >= 0 ? sB + sl * G::STOT : nullptr,
@@ -940,48 +1029,110 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
             if (a.hyp_order == 5) faces(std::true_type{});
             else faces(std::false_type{});
         }
+        // the next group's first values and the own cells' rates and old values of the
+        // group's first species, fetched before the barrier
+        const int g1 = g0 + GRP, gn1 = g1 < nfl ? (nfl - g1 < GRP ? nfl - g1 : GRP) : 0;
+        double pv[PF];
+        if (stab && gn1 > 0) {
+#pragma unroll
+            for (int k = 0; k < PF; k++) pv[k] = stage_load(g1, gn1, tid + k * NTH);
+        }
+        constexpr int NO = (G::NCELL + NTH - 1) / NTH, NP = kOne && GRP > 1 ? 2 : 1;
+        double pr[NO][NP], ps[NO][NP];
+        // (FP64: the old value is staged as it is, at the cell's place on its x line)
+        auto old_value = [&](const Own& w, int j) -> double {
+            if constexpr (PREC == PREC_FP64)
+                return sU[j * G::STOT + w.cx + 3 + G::template SE<0>(0) * (w.cy + G::template SE<0>(1) * w.cz)] * uisc;
+            else
+                return state(w, a.fl_sp[g0 + j]);
+        };
+#pragma unroll
+        for (int o = 0; o < NO; o++) {
+            Own w;
+            if constexpr (kOne) w = own1;
+            else w = own_cell(tid + o * NTH);
+#pragma unroll
+            for (int j = 0; j < NP; j++) {
+                pr[o][j] = ps[o][j] = 0.0;
+                if (w.ok && j < gn) {
+                    pr[o][j] = rate(w, a.fl_sp[g0 + j]);
+                    ps[o][j] = old_value(w, j);
+                }
+            }
+        }
         __syncthreads();
         // (3) divergence + sources of the own cell: dsdt = (Fx_lo - Fx_hi)/dx + rxn,
         // then += y and z terms (Source/ScalarSolve.cpp:45-51)
-        if (own) {
+        {
             // the own cell's dsdt of species j of the group, with its rate r, in the
             // reference's order: x faces + rate, then y, then z
             // (Source/ScalarSolve.cpp:45-51)
-            auto divergence = [&](int j, double r) -> double {
+            auto divergence = [&](const Own& w, int j, double r) -> double {
                 const VT* Fj = sF + j * G::FTOT;
                 double acc;
                 {
                     constexpr int F0 = G::template FE<0>(0), F1 = G::template FE<0>(1);
-                    const int lo_f = cx + F0 * (cy + F1 * cz);
-                    acc = ((double)Fj[lo_f] - (double)Fj[lo_f + 1]) * a.idx[0] + r;
+                    const int lo_f = w.cx + F0 * (w.cy + F1 * w.cz);
+                    acc = ((double)Fj[lo_f] - (double)Fj[lo_f + 1]) * (PREC == PREC_FP64 ? a.idx[0] * uisc : a.idx[0]) + r;
                 }
                 if constexpr (DIM > 1) {
                     constexpr int F0 = G::template FE<1>(0), F1 = G::template FE<1>(1);
-                    const int lo_f = G::FOFF1 + cx + F0 * (cy + F1 * cz);
-                    acc += ((double)Fj[lo_f] - (double)Fj[lo_f + F0]) * a.idx[1];
+                    const int lo_f = G::FOFF1 + w.cx + F0 * (w.cy + F1 * w.cz);
+                    acc += ((double)Fj[lo_f] - (double)Fj[lo_f + F0]) * (PREC == PREC_FP64 ? a.idx[1] * uisc : a.idx[1]);
                 }
                 if constexpr (DIM > 2) {
                     constexpr int F0 = G::template FE<2>(0), F1 = G::template FE<2>(1);
-                    const int lo_f = G::FOFF2 + cx + F0 * (cy + F1 * cz);
-                    acc += ((double)Fj[lo_f] - (double)Fj[lo_f + F0 * F1]) * a.idx[2];
+                    const int lo_f = G::FOFF2 + w.cx + F0 * (w.cy + F1 * w.cz);
+                    acc += ((double)Fj[lo_f] - (double)Fj[lo_f + F0 * F1]) * (PREC == PREC_FP64 ? a.idx[2] * uisc : a.idx[2]);
                 }
                 return acc;
             };
-            // two species at a time: their four loads in flight together
+            auto finish_one = [&](Own& w, int j, double r, double st) { finish(w, a.fl_sp[g0 + j], divergence(w, j, r), st); };
+            // two species at a time, the next two's loads in flight meanwhile
+            if constexpr (kOne) {
+                if (own1.ok) {
 #pragma unroll 1
-            for (int j = 0; j < gn; j += 2) {
-                const bool two = j + 1 < gn;
-                const int s0 = a.fl_sp[g0 + j], s1 = two ? a.fl_sp[g0 + j + 1] : s0;
-                const double r0 = rate(s0), r1 = rate(s1), st0 = state(s0), st1 = state(s1);
-                finish(s0, divergence(j, r0), st0);
-                if (two) finish(s1, divergence(j + 1, r1), st1);
+                    for (int j = 0; j < gn; j += NP) {
+                        double r[NP], st[NP];
+#pragma unroll
+                        for (int q = 0; q < NP; q++) {
+                            r[q] = pr[0][q];
+                            st[q] = ps[0][q];
+                            if (j + NP + q < gn) {
+                                pr[0][q] = rate(own1, a.fl_sp[g0 + j + NP + q]);
+                                ps[0][q] = old_value(own1, j + NP + q);
+                            }
+                        }
+#pragma unroll
+                        for (int q = 0; q < NP; q++)
+                            if (j + q < gn) finish_one(own1, j + q, r[q], st[q]);
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int o = 0; o < NO; o++) {
+                    Own w = own_cell(tid + o * NTH);
+                    if (!w.ok) continue;
+                    finish_one(w, 0, pr[o][0], ps[o][0]);
+#pragma unroll 1
+                    for (int j = 1; j < gn; j++) finish_one(w, j, rate(w, a.fl_sp[g0 + j]), old_value(w, j));
+                }
             }
         }
-        // the next group's staging overwrites sU only after every thread has passed
-        // the barrier above; sF is rewritten only after the next staging barrier,
-        // by which time every divergence read of this group is done
+        if (gn1 > 0) {
+            // FP64 old values of later species are read from the staged densities above
+            if (PREC == PREC_FP64 && GRP > 1) __syncthreads();
+            if (!stab) {
+                stage_far(g1, gn1);
+            } else {
+#pragma unroll
+                for (int k = 0; k < PF; k++) stage_store(gn1, tid + k * NTH, pv[k]);
+                stage_rest(g1, gn1, PF);
+            }
+            __syncthreads();  // the staged group is complete, and every read of sF is done
+        }
     }
-    if (own) {
+    each_own([&](Own& w) {
         // four species at a time: their loads in flight together
         constexpr int CH = 4;
 #pragma unroll 1
@@ -990,12 +1141,12 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
 #pragma unroll
             for (int k = 0; k < CH; k++) {
                 const int s = a.nf_sp[j0 + k < a.nnf ? j0 + k : a.nnf - 1];
-                r[k] = rate(s);
-                st[k] = state(s);
+                r[k] = rate(w, s);
+                st[k] = state(w, s);
             }
 #pragma unroll
             for (int k = 0; k < CH; k++)
-                if (j0 + k < a.nnf) finish(a.nf_sp[j0 + k], r[k], st[k]);
+                if (j0 + k < a.nnf) finish(w, a.nf_sp[j0 + k], r[k], st[k]);
         }
 #pragma unroll 1
         for (int j0 = 0; j0 < a.nbg; j0 += CH) {
@@ -1003,8 +1154,8 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
 #pragma unroll
             for (int k = 0; k < CH; k++) {
                 const int s = a.bg_sp[j0 + k < a.nbg ? j0 + k : a.nbg - 1];
-                r[k] = rate(s);
-                v[k] = state(s);
+                r[k] = rate(w, s);
+                v[k] = state(w, s);
             }
 #pragma unroll
             for (int k = 0; k < CH; k++) {
@@ -1015,20 +1166,23 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
                     if (v[k] < a.min_spec && a.bound_specden) v[k] = a.min_spec;
                 }
                 bad |= !isfinite(v[k]);
-                a.pn(gi, gj, gk, s) = v[k];
-                if (a.dsdt.p) a.dsdt(gi, gj, gk, s) = r[k];
+                out(w, s) = v[k];
+                if (a.dsdt.p) a.dsdt(w.gi, w.gj, w.gk, s) = r[k];
             }
         }
         if (a.update_te && a.elecenergy) {
             // Source/ScalarSolve.cpp:659-666
-            double te = (2.0 / 3.0) / K_B * een_new / state(a.e_id);
+            // (several own cells: the thread's own results, read back)
+            const double ne_new = kOne ? w.ne_new : out(w, a.e_id);
+            const double een_new = kOne ? w.een_new : out(w, VD_EEN(ns));
+            double te = (2.0 / 3.0) / K_B * een_new / state(w, a.e_id);
             if (te < a.min_te) {
                 te = a.min_te;
-                a.pn(gi, gj, gk, VD_EEN(ns)) = 1.5 * K_B * ne_new * te;
+                out(w, VD_EEN(ns)) = 1.5 * K_B * ne_new * te;
             }
-            a.pn(gi, gj, gk, VD_ETEMP(ns)) = te;
+            out(w, VD_ETEMP(ns)) = te;
         }
-    }
+    });
     if (a.status) {  // uniform over the CTA; every lane of every warp reaches it
         const unsigned any = __ballot_sync(0xffffffffu, bad);
         if (any && (threadIdx.x & 31) == 0) atomicOr(a.status, 1u);
@@ -1037,10 +1191,10 @@ __device__ __forceinline__ void transport_tile_update(const TransportArgs& a, in
 
 // per-box kernel: one CTA per tile
 template <int DIM, int PREC, int MINB>
-__global__ void __launch_bounds__(default_nth<DIM>(), MINB) k_transport(const __grid_constant__ TransportArgs a)
+__global__ void __launch_bounds__(default_nth<DIM, PREC>(), MINB) k_transport(const __grid_constant__ TransportArgs a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    using TS = typename DefaultTile<DIM>::T;
+    using TS = typename DefaultTile<DIM, PREC>::T;
     transport_tile_update<DIM, PREC, TS, group_fit<DIM, PREC, TS, MINB>()>(a, blockIdx.x, smem_raw);
 }
 
@@ -1056,6 +1210,7 @@ __global__ void __launch_bounds__(TS::NTH, MINB)
                       const BatchCtl ctl)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int NTH = TS::NTH;
     constexpr int NW = (int)(sizeof(TransportArgs) / 8);
     static_assert(sizeof(TransportArgs) % 8 == 0, "record copied in 8-byte words");
     __shared__ __align__(16) long long sA_raw[2][NW];
@@ -1068,7 +1223,7 @@ __global__ void __launch_bounds__(TS::NTH, MINB)
     };
     auto fetch = [&](int buf, int rec) {
         const long long* src = reinterpret_cast<const long long*>(boxes + rec);
-        for (int q = threadIdx.x; q < NW; q += TS::NTH) {
+        for (int q = threadIdx.x; q < NW; q += NTH) {
             const unsigned dst = (unsigned)__cvta_generic_to_shared(&sA_raw[buf][q]);
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src + q) : "memory");
         }
