@@ -35,6 +35,14 @@ std::string hexd(double x)
     return b;
 }
 
+std::string a_lit(double x)
+{
+    char b[64];
+    snprintf(b, sizeof(b), "%a", x);
+    return b;
+}
+
+constexpr int kRateChunk = 24, kRateUnroll = 8;
 // Layout-identical device-side definitions of A4 and PrepArgs (vd_types.cuh,
 // vd_kernels.cuh); the host checks sizeof(PrepArgs) against the value the
 // generated code reports through vd_spec_sizeof.
@@ -67,11 +75,9 @@ extern "C" __global__ void vd_spec_sizeof(unsigned long long* out)
     out[0] = sizeof(PrepArgs);
     out[1] = sizeof(BatchCtl);
 }
-// The FP64 rate exponential, called out of line: inlined, its instructions
-// repeated for every reaction made the straight-line chemistry overflow the
-// instruction cache (stall "no instruction"); out of line the FP64 prep kernel of
-// 150 reactions ran 10 % faster on B200, with bit-identical results.  The mixed
-// path's exp2 stays inline (out of line it was slower).
+// The FP64 exponential of the rates outside the table, called out of line: inlined
+// per reaction, its instructions made the straight-line chemistry overflow the
+// instruction cache (bit-identical results).
 __device__ __noinline__ double vd_exp64(double x) { return exp(x); }
 // 2^x as FP32 from an FP64 exponent (same as exp2_split in vd_device.cuh)
 __device__ __forceinline__ float exp2_split(double x)
@@ -136,13 +142,59 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
     std::ostringstream o;
     // minimum resident blocks per SM (caps registers at 65536 / (128 * min)); 0 leaves
     // the choice to the compiler.  VD_SPEC_MINBLOCKS overrides it for tuning.
-    // Default: about 4 registers per species plus 48 (FP64) or plus 32 (mixed: the
-    // rates are FP32), measured best on B200 for the 8- and 24-species mechanisms
-    // (FP64: 6 and 3 blocks of 128 threads per SM; mixed: 8 and 4).
-    int minb = 65536 / (128 * (4 * ns + (prec == PREC_MIXED ? 32 : 48)));
+    // Default: about 4 registers per species plus 32, measured best on B200 for the
+    // 8- and 24-species mechanisms (8 and 4 blocks of 128 threads per SM).
+    int minb = 65536 / (128 * (4 * ns + 32));
     minb = minb < 1 ? 1 : (minb > 8 ? 8 : minb);
     if (const char* e = getenv("VD_SPEC_MINBLOCKS")) minb = atoi(e);
     const std::string sfx = prec == PREC_MIXED ? "mixed" : "fp64";
+    // Rates of the Arrhenius-in-Te reactions go through a rolled loop over a table in
+    // constant memory, kRateChunk at a time, into the thread's column of a shared
+    // array, ahead of the straight-line code that uses them: the exponentials of
+    // several reactions are then independent work in flight and their code is there
+    // once per chunk.  FP64, 24 species and 150 reactions on 128^3, B200: 1.26 ms
+    // with the exponential called out of line per reaction, 1.13 ms rolled, 24 at a
+    // time unrolled by 8, at 3 blocks per SM and 1.04 ms at 4 (16 at a time unrolled
+    // by 4 1.18 ms at 3 blocks; concentrations in shared memory 1.07 ms at 4).
+    // Bound by the latency of FP64 chains at 16 warps per SM (FP64 pipe 47 %).
+    const int rate_bytes = prec == PREC_MIXED ? 4 : 8;
+    int kchunk = 200 * 1024 / (128 * rate_bytes * (minb > 0 ? minb : 1)) / 4 * 4;
+    kchunk = kchunk > kRateChunk ? kRateChunk : kchunk;
+    auto in_table = [&](const VdRxnDev& R) { return R.kind == VD_RATE_ARRHENIUS_TE && R.A > 0.0; };
+    struct Chunk {
+        int r0, r1, t0, n;  // reactions [r0, r1) with n table entries from t0 (padded to fours)
+    };
+    std::vector<Chunk> chunks;
+    {
+        std::ostringstream tab;
+        int t = 0, nt = 0;
+        Chunk c{0, 0, 0, 0};
+        auto entry = [&](double a, double b, double d) {
+            tab << (nt ? ", " : "") << a_lit(a) << ", " << a_lit(b) << ", " << a_lit(d);
+            nt++;
+        };
+        for (int r = 0; r < m.nr; r++) {
+            const VdRxnDev& R = m.rxn[r];
+            if (in_table(R)) {
+                if (c.n == kchunk) {
+                    c.r1 = r;
+                    chunks.push_back(c);
+                    t = nt;
+                    c = Chunk{r, 0, t, 0};
+                }
+                if (prec == PREC_MIXED) entry(R.l2A, R.b, R.Cl2);
+                else entry(R.lnA, R.b, R.C);
+                c.n++;
+            }
+        }
+        while (nt % 4) entry(0.0, 0.0, 0.0);
+        c.r1 = m.nr;
+        chunks.push_back(c);
+        int most = 0;
+        for (const Chunk& q : chunks) most = q.n > most ? q.n : most;
+        kchunk = (most + 3) / 4 * 4;  // columns of the shared array
+        if (nt) o << "__constant__ double vd_rates_" << sfx << "[" << 3 * nt << "] = {" << tab.str() << "};\n";
+    }
     const std::string lb = "__launch_bounds__(128" + (minb > 0 ? ", " + std::to_string(minb) : std::string()) + ")";
     // per-box kernel (grid-stride over the grown box) and batched kernel (work list
     // of (box, chunk of kPrepChunk cells)), both around one per-cell function
@@ -174,6 +226,9 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
       << "      if (idx < ntot) vd_spec_cell_" << sfx << "(a, idx);\n"
       << "    }\n  }\n}\n";
     o << "__device__ __forceinline__ void vd_spec_cell_" << sfx << "(const PrepArgs& a, i64 idx)\n{\n";
+    if (kchunk > 0 && chunks[0].n > 0)
+        o << "  __shared__ " << (prec == PREC_MIXED ? "float" : "double") << " ks_all[" << 128 * kchunk << "];\n"
+          << "  " << (prec == PREC_MIXED ? "float" : "double") << "* const ks = ks_all + threadIdx.x;\n";
     o << "  const double N_A = " << hexd(N_A) << ", NA_CE = " << hexd(NA_CE) << ", KB_CE = " << hexd(KB_CE)
       << ", K_B = " << hexd(K_B) << ";\n";
     o << "  const int gx = a.ghi[0] - a.glo[0] + 1, gy = a.ghi[1] - a.glo[1] + 1;\n"
@@ -249,10 +304,27 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
             o << "        k = (double)exp2_split(fma(sum, " << hexd(1.4426950408889634074) << ", "
               << hexd(janev ? F.l2jA : F.l2fA) << "));\n";
     };
+    size_t ci = 0;
+    int kk = 0;
     for (int r = 0; r < m.nr; r++) {
         const VdRxnDev& R = m.rxn[r];
+        if (ci < chunks.size() && r == chunks[ci].r0) {
+            const Chunk& c = chunks[ci++];
+            kk = 0;
+            if (c.n > 0) {
+                const int n4 = (c.n + 3) / 4 * 4;
+                o << "#pragma unroll " << kRateUnroll << "\n    for (int t = 0; t < " << n4 << "; t++) {\n"
+                  << "      const double* rt = vd_rates_" << sfx << " + 3 * (" << c.t0 << " + t);\n";
+                if (prec == PREC_MIXED)
+                    o << "      ks[t * 128] = exp2_split(fma(rt[1], lTe, rt[0]) - rt[2] * invTe);\n    }\n";
+                else
+                    o << "      ks[t * 128] = exp(fma(rt[1], lTe, rt[0]) - rt[2] * invTe);\n    }\n";
+            }
+        }
         o << "    { // reaction " << r << "\n      double k;\n";
-        if (R.kind == VD_RATE_CONST) {
+        if (in_table(R)) {
+            o << "      k = (double)ks[" << 128 * kk++ << "];\n";
+        } else if (R.kind == VD_RATE_CONST) {
             o << "      k = " << hexd(R.A) << ";\n";
         } else if (R.kind == VD_RATE_TOWNSEND) {
             const double* c = m.fits[R.fit].jc;
