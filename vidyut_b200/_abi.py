@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import struct
 from pathlib import Path
 
 MAX_SPECIES = 64
@@ -190,31 +191,33 @@ def check(status: int, where: str) -> None:
 
 
 def make_box(lo, hi, dim: int) -> VdBox:
-    b = VdBox()
-    for d in range(3):
-        b.lo[d] = int(lo[d]) if d < len(lo) else 0
-        b.hi[d] = int(hi[d]) if d < len(hi) else 0
-        b.itype[d] = 0
-    b.dim = dim
-    return b
+    if len(lo) < 3 or len(hi) < 3:
+        lo, hi = (*lo, 0, 0, 0), (*hi, 0, 0, 0)
+    return VdBox.from_buffer_copy(_PACK_BOX(int(lo[0]), int(lo[1]), int(lo[2]), int(hi[0]), int(hi[1]), int(hi[2]),
+                                            0, 0, 0, dim))
+
+
+_PACK_BOX = struct.Struct("@10i").pack
 
 
 def make_array4(ptr: int, shape, begin, ncomp: int | None = None) -> VdArray4:
     """Array4 over a C-ordered buffer of shape (ncomp, nz, ny, nx) whose element
     [n, 0, 0, 0] is cell (begin[0], begin[1], begin[2])."""
+    return VdArray4.from_buffer_copy(pack_array4(ptr, shape, begin, ncomp))
+
+
+# The fields of a VdArray4 packed in one call: setting them one by one through ctypes
+# took 3 us per array, most of the host time of a small box's update (a dozen arrays).
+_PACK_A4 = struct.Struct("@Pqqqiiiiiii4x").pack
+assert struct.calcsize("@Pqqqiiiiiii4x") == C.sizeof(VdArray4)
+A4x3 = VdArray4 * 3
+
+
+def pack_array4(ptr: int, shape, begin, ncomp: int | None = None) -> bytes:
     nc, nz, ny, nx = shape
-    a = VdArray4()
-    a.p = ptr
-    a.jstride = nx
-    a.kstride = nx * ny
-    a.nstride = nx * ny * nz
-    for d in range(3):
-        a.begin[d] = int(begin[d])
-    a.end[0] = begin[0] + nx
-    a.end[1] = begin[1] + ny
-    a.end[2] = begin[2] + nz
-    a.ncomp = nc if ncomp is None else ncomp
-    return a
+    bx, by, bz = begin
+    js = nx * ny
+    return _PACK_A4(ptr, nx, js, js * nz, bx, by, bz, bx + nx, by + ny, bz + nz, nc if ncomp is None else ncomp)
 
 
 def null_array4() -> VdArray4:
