@@ -527,8 +527,14 @@ int vd_compute_explicit_flux(const vd_box* bx, int dir, int specid, vd_array4 ph
     if (user_vel)
         for (int d = 0; d < 3; d++) uv[d] = user_vel[d];
     int dl[3] = {domlo[0], domlo[1], domlo[2]}, dh[3] = {domhi[0], domhi[1], domhi[2]};
+    int mk;  // the species' mobility model (a scaled one: its reference's)
+    {
+        std::lock_guard<std::mutex> lk(g_mech_mu);
+        mk = g_mech->mob_kind[specid];
+        if (mk == VD_MOB_SCALED) mk = g_mech->mob_kind[g_mech->mob_ref[specid]];
+    }
     cudaError_t e = launch_face_flux(box_idx(flo, fhi), dir, specid, A4(phi), A4(fx), zlo, zhi, dl, dh, Tg, dxmin,
-                                     dt, hyp_order, user_defined_vel, weno_scheme, uv, vel_species, ns, st);
+                                     dt, hyp_order, user_defined_vel, weno_scheme, uv, vel_species, ns, mk, st);
     if (e != cudaSuccess) return cuda_fail(e, "k_face_flux launch");
     return VD_OK;
 }

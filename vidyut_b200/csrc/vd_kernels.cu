@@ -180,6 +180,22 @@ static cudaError_t chem_smem(const void* fn, int ns, int threads, size_t* bytes)
 cudaError_t launch_reaction_source(const BoxIdx& b, const A4& sb, const A4& rxn, double Tg, int prec, int ns,
                                    cudaStream_t st)
 {
+    if (prec == PREC_FP64) {
+        // the generated chemistry over the valid box: the table-driven kernel's bits at
+        // a third of its time (64^3, 12 species / 60 reactions: 198 -> 56 us)
+        PrepArgs pa;
+        memset((void*)&pa, 0, sizeof(pa));
+        pa.sb = sb;
+        pa.rxn = rxn;
+        for (int d = 0; d < 3; d++) {
+            pa.glo[d] = pa.lo[d] = b.lo[d];
+            pa.ghi[d] = pa.hi[d] = b.hi[d];
+        }
+        pa.Tg = Tg;
+        pa.do_reactions = 1;
+        cudaError_t es = spec_launch_source(pa, st);
+        if (es != cudaErrorNotReady) return es;
+    }
     unsigned g = grid_for(b.ncell, 128);
     size_t sm = 0;
     const void* fn = prec == PREC_MIXED ? (const void*)k_reaction_source<PREC_MIXED>
@@ -193,74 +209,127 @@ cudaError_t launch_reaction_source(const BoxIdx& b, const A4& sb, const A4& rxn,
 }
 
 // ---------------------------------------------------------------------------
-// velocity of species s at cell (i,j,k) in direction d (plasmachem_transport::compute_vel,
-// Source/PlasmaChem.H:187-206, or the constant user velocity of the Advect case)
-__device__ __forceinline__ double vel_cell(const A4& phi, int i, int j, int k, int d, int s, int ns, double Tg,
-                                           int udv, const double* uvel, int vel_sp)
-{
-    if (udv) return (s == vel_sp) ? uvel[d] : 0.0;
-    const int64_t o = phi.off(i, j, k);
-    double N = 0.0;
-    for (int q = 0; q < ns; q++) N += phi.p[o + q * phi.ns];
-    double Te = phi.p[o + (int64_t)VD_ETEMP(ns) * phi.ns];
-    // |E| of the three state components, as compute_vel takes it
-    double esum = 0.0;
-    for (int q = 0; q < 3; q++) {
-        const double e = phi.p[o + (int64_t)(VD_EFX(ns) + q) * phi.ns];
-        esum += e * e;
-    }
-    double mu = mob_fp64(s, Te, N, Tg, sqrt(esum));
-    return mu * phi.p[o + (int64_t)(VD_EFX(ns) + d) * phi.ns];
-}
-
+// One species' face fluxes in one direction.  A CTA takes a tile of faces: L along the
+// sweep direction DIR by W across it (x across for DIR 1 and 2, rows for DIR 0).  The
+// density and the velocity of every cell of the tile's stencil lines are staged once
+// in shared memory -- the velocity needs the sum over all species of a cell
+// (plasmachem_transport::compute_vel, Source/PlasmaChem.H:187-206, or the constant
+// user velocity of the Advect case), which one thread per face made for each of its
+// six cells -- then each thread evaluates its faces from there.  Bound by the loads'
+// latency at small boxes, by the species sums' reads at large ones (event-timed, one
+// call: 256^2, 8 species 16.8 -> 9.8 us; 64^3, 12 species 39.7 -> 18.7 us).
 struct FaceFluxArgs {
     BoxIdx fb;
-    int dir, specid, ns;
+    int specid, ns;
     A4 phi, fx;
     int8_t zlo, zhi;
     int domlo, domhi;
     double Tg, dxmin, dt;
     int hyp_order, udv, weno, vel_sp;
-    double uvel[3];
+    double uvel;
+    // the velocity reads the density sum (a drifting species), |E| (a mobility model in
+    // the field); otherwise those loads are left out
+    int need_n, need_emag;
 };
 
-__global__ void __launch_bounds__(128) k_face_flux(const __grid_constant__ FaceFluxArgs a)
+template <int DIR, int L, int W>
+__global__ void __launch_bounds__(256) k_face_flux(const __grid_constant__ FaceFluxArgs a)
 {
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < a.fb.ncell;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int c[3];
-        cell_of(a.fb, idx, c[0], c[1], c[2]);
-        double u[6], v[6];
-        const int H = (a.hyp_order == 5) ? 3 : a.hyp_order;
-#pragma unroll
-        for (int q = 0; q < 6; q++) {
-            int off = q - 3;  // cells i-3 .. i+2 along dir
-            if (off < -H || off > H - 1) {
-                u[q] = 0.0;
-                v[q] = 0.0;
-                continue;
-            }
-            int g[3] = {c[0], c[1], c[2]};
-            g[a.dir] += off;
-            u[q] = a.phi(g[0], g[1], g[2], a.specid);
-            v[q] = vel_cell(a.phi, g[0], g[1], g[2], a.dir, a.specid, a.ns, a.Tg, a.udv, a.uvel, a.vel_sp);
+    constexpr int NC = L + 5;  // cells f0 - 3 .. f0 + L + 1 of a line
+    __shared__ double su[NC * W], sv[NC * W];
+    const int H = a.hyp_order == 5 ? 3 : a.hyp_order;
+    // tile origin: faces f0 .. f0 + L - 1 along DIR, transverse positions from t0
+    int f0, t0, t1 = 0;  // t0: x (DIR 1, 2) or row j + ny k (DIR 0); t1: the other transverse index
+    const int rows = a.fb.n[1] * a.fb.n[2];
+    t0 = blockIdx.x * W;
+    f0 = blockIdx.y * L;
+    const int nt = DIR == 0 ? rows : a.fb.n[0];
+    // offset (from the face box's low corner) of line position p = f - f0 .. and
+    // transverse position w
+    auto cell = [&](int f, int w, int* g) {
+        if (DIR == 0) {
+            const int r = t0 + w;
+            g[0] = f;
+            g[2] = r / a.fb.n[1];
+            g[1] = r - g[2] * a.fb.n[1];
+        } else if (DIR == 1) {
+            g[0] = t0 + w;
+            g[1] = f;
+            g[2] = t1;
+        } else {
+            g[0] = t0 + w;
+            g[1] = t1;
+            g[2] = f;
         }
-        double F = face_flux_fp64(u, v, a.hyp_order, a.weno, a.dxmin, a.dt);
-        int fd = c[a.dir];
-        if (fd == a.domlo && a.zlo) F = 0.0;
-        if (fd == a.domhi + 1 && a.zhi) F = 0.0;
-        a.fx(c[0], c[1], c[2], 0) = F;
+        for (int e = 0; e < 3; e++) g[e] += a.fb.lo[e];
+    };
+    const int ns = a.ns;
+    const int64_t cs = a.phi.ns;
+    const int nt1 = DIR == 0 ? 1 : a.fb.n[DIR == 1 ? 2 : 1];
+    for (t1 = blockIdx.z; t1 < nt1; t1 += gridDim.z) {
+        if (t1 != (int)blockIdx.z) __syncthreads();  // the staged cells are read by others until here
+        for (int q = threadIdx.x; q < NC * W; q += 256) {
+            const int w = DIR == 0 ? q / NC : q % W, c = DIR == 0 ? q % NC : q / W;
+            const int f = f0 + c - 3;  // cell f lies above face f; the box's stencil spans -H .. n - 2 + H
+            double u = 0.0, v = 0.0;
+            if (t0 + w < nt && f >= -H && f <= a.fb.n[DIR] - 2 + H) {
+                int g[3];
+                cell(f, w, g);
+                const double* p = a.phi.p + a.phi.off(g[0], g[1], g[2]);
+                u = __ldg(p + a.specid * cs);
+                if (a.udv) {
+                    v = a.specid == a.vel_sp ? a.uvel : 0.0;
+                } else {
+                    const double E = __ldg(p + (VD_EFX(ns) + DIR) * cs);
+                    double N = 0.0, Te = 0.0, esum = 0.0;
+                    if (a.need_n) {
+                        Te = __ldg(p + VD_ETEMP(ns) * cs);
+#pragma unroll 8
+                        for (int s = 0; s < ns; s++) N += __ldg(p + s * cs);
+                    }
+                    if (a.need_emag) {
+                        // |E| of the three state components, as compute_vel takes it
+                        for (int e = 0; e < 3; e++) {
+                            const double x = __ldg(p + (VD_EFX(ns) + e) * cs);
+                            esum += x * x;
+                        }
+                    }
+                    v = mob_fp64(a.specid, Te, N, a.Tg, sqrt(esum)) * E;
+                }
+            }
+            su[q] = u;
+            sv[q] = v;
+        }
+        __syncthreads();
+        constexpr int STR = DIR == 0 ? 1 : W;
+        for (int q = threadIdx.x; q < L * W; q += 256) {
+            const int w = DIR == 0 ? q / L : q % W, c = DIR == 0 ? q % L : q / W;
+            const int f = f0 + c;
+            if (t0 + w >= nt || f >= a.fb.n[DIR]) continue;
+            double u[6], v[6];
+            const int base = DIR == 0 ? w * NC + c : q;
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                u[k] = su[base + k * STR];
+                v[k] = sv[base + k * STR];
+            }
+            double F = face_flux_fp64(u, v, a.hyp_order, a.weno, a.dxmin, a.dt);
+            int g[3];
+            cell(f, w, g);
+            if (g[DIR] == a.domlo && a.zlo) F = 0.0;
+            if (g[DIR] == a.domhi + 1 && a.zhi) F = 0.0;
+            a.fx.p[a.fx.off(g[0], g[1], g[2])] = F;
+        }
     }
 }
 
 cudaError_t launch_face_flux(const BoxIdx& fb, int dir, int specid, const A4& phi, const A4& fx,
                              const int8_t zlo[3], const int8_t zhi[3], const int domlo[3], const int domhi[3],
                              double Tg, double dxmin, double dt, int hyp_order, int udv, int weno,
-                             const double uvel[3], int vel_sp, int ns, cudaStream_t st)
+                             const double uvel[3], int vel_sp, int ns, int mob_kind, cudaStream_t st)
 {
     FaceFluxArgs a;
     a.fb = fb;
-    a.dir = dir;
     a.specid = specid;
     a.ns = ns;
     a.phi = phi;
@@ -276,20 +345,38 @@ cudaError_t launch_face_flux(const BoxIdx& fb, int dir, int specid, const A4& ph
     a.udv = udv;
     a.weno = weno;
     a.vel_sp = vel_sp;
-    for (int d = 0; d < 3; d++) a.uvel[d] = uvel[d];
+    a.uvel = uvel[dir];
+    a.need_n = mob_kind != VD_MOB_ZERO;
+    a.need_emag = mob_kind == VD_MOB_POW_EMAG || mob_kind == VD_MOB_EN_POLY;
     ProfScope ps("k_face_flux", st);
-    k_face_flux<<<grid_for(fb.ncell, 128), 128, 0, st>>>(a);
+    const auto up = [](int64_t n, int t) { return (unsigned)((n + t - 1) / t); };
+    const auto zdim = [](int n) { return (unsigned)(n < 65535 ? n : 65535); };
+    // tiles of 256 faces; along y and z of 512 when that still gives every SM a CTA
+    // (1.3 staged cells per face instead of 1.6)
+    const bool tall = (int64_t)up(fb.n[0], 32) * up(fb.n[dir], 16) * fb.n[dir == 1 ? 2 : 1] >= 2 * 148;
+    if (dir == 0) {
+        k_face_flux<0, 32, 8><<<dim3(up((int64_t)fb.n[1] * fb.n[2], 8), up(fb.n[0], 32)), 256, 0, st>>>(a);
+    } else if (dir == 1) {
+        if (tall) k_face_flux<1, 16, 32><<<dim3(up(fb.n[0], 32), up(fb.n[1], 16), zdim(fb.n[2])), 256, 0, st>>>(a);
+        else k_face_flux<1, 8, 32><<<dim3(up(fb.n[0], 32), up(fb.n[1], 8), zdim(fb.n[2])), 256, 0, st>>>(a);
+    } else {
+        if (tall) k_face_flux<2, 16, 32><<<dim3(up(fb.n[0], 32), up(fb.n[2], 16), zdim(fb.n[1])), 256, 0, st>>>(a);
+        else k_face_flux<2, 8, 32><<<dim3(up(fb.n[0], 32), up(fb.n[2], 8), zdim(fb.n[1])), 256, 0, st>>>(a);
+    }
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_dsdt(BoxIdx b, int dim, int specid, A4 f0, A4 f1, A4 f2, A4 rxn, A4 dsdt,
+// x over the threads, rows (j, k) over the blocks: no index division per cell
+__global__ void __launch_bounds__(128) k_dsdt(BoxIdx b, int dim, int specid, A4 f0, A4 f1, A4 f2, A4 rxn, A4 dsdt,
                                               double dx0, double dx1, double dx2)
 {
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < b.ncell;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_of(b, idx, i, j, k);
+    const int ii = blockIdx.x * 128 + threadIdx.x;
+    if (ii >= b.n[0]) return;
+    const int i = b.lo[0] + ii;
+    for (int r = blockIdx.y; r < b.n[1] * b.n[2]; r += gridDim.y) {
+        const int kk = r / b.n[1];
+        const int j = b.lo[1] + r - kk * b.n[1], k = b.lo[2] + kk;
         double v = (f0(i, j, k) - f0(i + 1, j, k)) / dx0 + rxn(i, j, k, specid);
         if (dim > 1) v += (f1(i, j, k) - f1(i, j + 1, k)) / dx1;
         if (dim == 3) v += (f2(i, j, k) - f2(i, j, k + 1)) / dx2;
@@ -301,22 +388,52 @@ cudaError_t launch_dsdt(const BoxIdx& b, int dim, int specid, const A4 flux[3], 
                         const double dx[3], cudaStream_t st)
 {
     ProfScope ps("k_dsdt", st);
-    k_dsdt<<<grid_for(b.ncell, 256), 256, 0, st>>>(b, dim, specid, flux[0], flux[1], flux[2], rxn, dsdt, dx[0],
-                                                    dx[1], dx[2]);
+    const int64_t rows = (int64_t)b.n[1] * b.n[2];
+    const dim3 g((unsigned)((b.n[0] + 127) / 128), (unsigned)(rows < 65535 ? rows : 65535));
+    k_dsdt<<<g, 128, 0, st>>>(b, dim, specid, flux[0], flux[1], flux[2], rxn, dsdt, dx[0], dx[1], dx[2]);
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(128) k_joule(BoxIdx b, int dim, const __grid_constant__ TransportArgs a)
+// The Joule term as a call of its own: the density sums of the tile's cells and of the
+// cells around it once each into shared memory (every face reads two of them), then
+// joule_cell per cell.
+template <int DIM>
+__global__ void __launch_bounds__(kJouleThreads) k_joule(const __grid_constant__ TransportArgs a, int64_t ntiles)
 {
+    using JT = JouleTile<DIM>;
+    constexpr int E0 = JT::X + 2, E1 = JT::Y + 2 * (DIM > 1), E2 = JT::Z + 2 * (DIM > 2);
+    __shared__ double sN[E0 * E1 * E2];
     const int ns = a.ns;
-    for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < b.ncell;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        int i, j, k;
-        cell_of(b, idx, i, j, k);
-        double jh = joule_cell<false>(a, dim, i, j, k);
-        a.dsdt(i, j, k) += jh;
-        a.pn(i, j, k, VD_EJH(ns)) = jh;
-        a.pn(i, j, k, VD_EIH(ns)) = a.rxn(i, j, k, ns);
+    const int nt0 = (a.hi[0] - a.lo[0] + JT::X) / JT::X, nt1 = (a.hi[1] - a.lo[1] + JT::Y) / JT::Y;
+    const int cx = threadIdx.x % JT::X, cy = (threadIdx.x / JT::X) % JT::Y, cz = threadIdx.x / (JT::X * JT::Y);
+    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const int tix = (int)(t % nt0), tr = (int)(t / nt0);
+        const int o0 = a.lo[0] + tix * JT::X, o1 = a.lo[1] + (tr % nt1) * JT::Y, o2 = a.lo[2] + (tr / nt1) * JT::Z;
+        for (int q = threadIdx.x; q < E0 * E1 * E2; q += kJouleThreads) {
+            const int i = o0 - 1 + q % E0, j = o1 - (DIM > 1) + (q / E0) % E1, k = o2 - (DIM > 2) + q / (E0 * E1);
+            double N = 0.0;
+            if (i <= a.hi[0] + 1 && j <= a.hi[1] + (DIM > 1) && k <= a.hi[2] + (DIM > 2)) {
+                const double* p = a.sb.p + a.sb.off(i, j, k);
+                // the corner cells of the tile's box are no face's: left out
+                const int out = (i < a.lo[0] || i > a.hi[0]) + (j < a.lo[1] || j > a.hi[1]) + (k < a.lo[2] || k > a.hi[2]);
+                if (out <= 1) {
+#pragma unroll 8
+                    for (int s = 0; s < ns; s++) N += __ldg(p + s * a.sb.ns);
+                }
+            }
+            sN[q] = N;
+        }
+        __syncthreads();
+        const int i = o0 + cx, j = o1 + cy, k = o2 + cz;
+        if (i <= a.hi[0] && j <= a.hi[1] && k <= a.hi[2]) {
+            const double jh = joule_cell(a, DIM, i, j, k, [&](int x, int y, int z) {
+                return sN[(x - o0 + 1) + E0 * ((y - o1 + (DIM > 1)) + E1 * (z - o2 + (DIM > 2)))];
+            });
+            a.dsdt(i, j, k) += jh;
+            a.pn(i, j, k, VD_EJH(ns)) = jh;
+            a.pn(i, j, k, VD_EIH(ns)) = a.rxn(i, j, k, ns);
+        }
+        __syncthreads();  // the next tile rewrites the sums
     }
 }
 
@@ -332,8 +449,18 @@ cudaError_t launch_joule(const BoxIdx& b, int dim, const A4& sb, const A4& rxn, 
         a.ef[d] = ef[d];
         a.gne[d] = gne[d];
     }
+    for (int d = 0; d < 3; d++) {
+        a.lo[d] = b.lo[d];
+        a.hi[d] = b.hi[d];
+    }
+    const int64_t nt = dim == 1   ? joule_tile_count<1>(a.lo, a.hi)
+                       : dim == 2 ? joule_tile_count<2>(a.lo, a.hi)
+                                  : joule_tile_count<3>(a.lo, a.hi);
+    const unsigned g = (unsigned)(nt < (1 << 30) ? nt : (1 << 30));
     ProfScope ps("k_joule", st);
-    k_joule<<<grid_for(b.ncell, 128), 128, 0, st>>>(b, dim, a);
+    if (dim == 1) k_joule<1><<<g, kJouleThreads, 0, st>>>(a, nt);
+    else if (dim == 2) k_joule<2><<<g, kJouleThreads, 0, st>>>(a, nt);
+    else k_joule<3><<<g, kJouleThreads, 0, st>>>(a, nt);
     return cudaGetLastError();
 }
 

@@ -142,7 +142,7 @@ cudaError_t launch_reaction_source(const BoxIdx& b, const A4& sb, const A4& rxn,
 cudaError_t launch_face_flux(const BoxIdx& fb, int dir, int specid, const A4& phi, const A4& fx,
                              const int8_t zlo[3], const int8_t zhi[3], const int domlo[3], const int domhi[3],
                              double Tg, double dxmin, double dt, int hyp_order, int udv, int weno,
-                             const double uvel[3], int vel_sp, int ns, cudaStream_t st);
+                             const double uvel[3], int vel_sp, int ns, int mob_kind, cudaStream_t st);
 cudaError_t launch_dsdt(const BoxIdx& b, int dim, int specid, const A4 flux[3], const A4& rxn, const A4& dsdt,
                         const double dx[3], cudaStream_t st);
 cudaError_t launch_joule(const BoxIdx& b, int dim, const A4& sb, const A4& rxn, const A4 ef[3], const A4 gne[3],
@@ -202,6 +202,7 @@ bool spec_active();
 void spec_set_enabled(bool on);
 const char* spec_error();
 cudaError_t spec_launch_prep(const PrepArgs& a, int prec, cudaStream_t st);
+cudaError_t spec_launch_source(const PrepArgs& a, cudaStream_t st);
 cudaError_t spec_launch_prep_batch(const PrepArgs* boxes, const int2* items, int nitems, BatchCtl ctl, int prec,
                                    cudaStream_t st);
 int spec_compile_only(const VdMechDev& m, size_t* cubin_bytes);

@@ -135,7 +135,12 @@ std::string mob_expr(const VdMechDev& m, int s, const char* Te, const char* nd, 
     return o.str();
 }
 
-std::string gen_prep_kernel(const VdMechDev& m, int prec)
+// source: the reaction source alone (vd_reaction_source, FP64), with each rate of
+// progress rounded before it is added, as the table-driven kernel has it: the compiler
+// otherwise contracts w + k prod into one operation where a coefficient is 1, which
+// moves a net rate that is a near-total cancellation (3e-10 of a species' largest
+// source for 12 species and 60 reactions).
+std::string gen_prep_kernel(const VdMechDev& m, int prec, bool source = false)
 {
     const int ns = m.ns;
     const int eid = m.e_id;
@@ -147,7 +152,7 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
     int minb = 65536 / (128 * (4 * ns + 32));
     minb = minb < 1 ? 1 : (minb > 8 ? 8 : minb);
     if (const char* e = getenv("VD_SPEC_MINBLOCKS")) minb = atoi(e);
-    const std::string sfx = prec == PREC_MIXED ? "mixed" : "fp64";
+    const std::string sfx = source ? "source" : prec == PREC_MIXED ? "mixed" : "fp64";
     // Rates of the Arrhenius-in-Te reactions go through a rolled loop over a table in
     // constant memory, kRateChunk at a time, into the thread's column of a shared
     // array, ahead of the straight-line code that uses them: the exponentials of
@@ -203,6 +208,7 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
       << "  const i64 ntot = (i64)(a.ghi[0] - a.glo[0] + 1) * (a.ghi[1] - a.glo[1] + 1) * (a.ghi[2] - a.glo[2] + 1);\n"
       << "  for (i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x; idx < ntot; idx += (i64)gridDim.x * blockDim.x)\n"
       << "    vd_spec_cell_" << sfx << "(a, idx);\n}\n";
+    if (!source)
     o << "extern \"C\" __global__ void " << lb << " vd_spec_prep_batch_" << sfx
       << "(const PrepArgs* __restrict__ boxes, const int2* __restrict__ items, int nitems, const BatchCtl ctl)\n{\n"
       << "  __shared__ PrepArgs a;  // the item's record\n"
@@ -359,9 +365,9 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec)
                   << hexd(R.Cl2) << " * " << iT << ");\n";
             }
         }
-        o << "      const double q = k * ";
+        o << (source ? "      const double q = __dmul_rn(k, " : "      const double q = k * ");
         for (int t = 0; t < R.nreac; t++) o << (t ? " * " : "(") << "sc" << (int)R.reac[t];
-        o << ");\n";
+        o << (source ? "));\n" : ");\n");
         for (int t = 0; t < R.nterms; t++)
             o << "      w" << (int)R.sp[t] << " = fma(" << hexd(R.coef[t]) << ", q, w" << (int)R.sp[t] << ");\n";
         if (R.rxntype == VD_RXN_EXCITATION || R.rxntype == VD_RXN_IONIZATION)
@@ -391,6 +397,7 @@ struct SpecModule {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t prep[2] = {nullptr, nullptr};
     cudaKernel_t batch[2] = {nullptr, nullptr};
+    cudaKernel_t source = nullptr;
 };
 
 std::mutex g_spec_mu;
@@ -427,7 +434,8 @@ int spec_build(const VdMechDev& m)
         g_spec_err = "specialisation switched off";
         return 1;
     }
-    std::string src = std::string(kPrelude) + gen_prep_kernel(m, PREC_FP64) + gen_prep_kernel(m, PREC_MIXED);
+    std::string src = std::string(kPrelude) + gen_prep_kernel(m, PREC_FP64) + gen_prep_kernel(m, PREC_MIXED) +
+                      gen_prep_kernel(m, PREC_FP64, true);
     auto it = g_cache.find(src);
     if (it != g_cache.end()) {
         g_active = it->second;
@@ -460,6 +468,7 @@ int spec_build(const VdMechDev& m)
     cudaError_t e = cudaLibraryLoadData(&mod->lib, bin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->prep[PREC_FP64], mod->lib, "vd_spec_prep_fp64");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->prep[PREC_MIXED], mod->lib, "vd_spec_prep_mixed");
+    if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->source, mod->lib, "vd_spec_prep_source");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->batch[PREC_FP64], mod->lib, "vd_spec_prep_batch_fp64");
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&mod->batch[PREC_MIXED], mod->lib, "vd_spec_prep_batch_mixed");
     if (e == cudaSuccess) {
@@ -499,7 +508,8 @@ int spec_build(const VdMechDev& m)
 // needs no GPU.  Returns 0 on success; spec_error() holds the NVRTC log otherwise.
 int spec_compile_only(const VdMechDev& m, size_t* cubin_bytes)
 {
-    std::string src = std::string(kPrelude) + gen_prep_kernel(m, PREC_FP64) + gen_prep_kernel(m, PREC_MIXED);
+    std::string src = std::string(kPrelude) + gen_prep_kernel(m, PREC_FP64) + gen_prep_kernel(m, PREC_MIXED) +
+                      gen_prep_kernel(m, PREC_FP64, true);
     nvrtcProgram prog;
     if (nvrtcCreateProgram(&prog, src.c_str(), "vd_spec_chem.cu", 0, nullptr, nullptr) != NVRTC_SUCCESS) {
         g_spec_err = "nvrtcCreateProgram failed";
@@ -525,6 +535,17 @@ int spec_compile_only(const VdMechDev& m, size_t* cubin_bytes)
 
 // Launch the specialised prep kernel if active; returns cudaErrorNotReady when the
 // table-driven kernel must be used instead.
+static cudaError_t launch_over(cudaKernel_t k, const PrepArgs& a, const char* name, cudaStream_t st)
+{
+    int64_t n = (int64_t)(a.ghi[0] - a.glo[0] + 1) * (a.ghi[1] - a.glo[1] + 1) * (a.ghi[2] - a.glo[2] + 1);
+    int64_t g = (n + 127) / 128;
+    if (g > 148LL * 64) g = 148LL * 64;
+    if (g < 1) g = 1;
+    PrepArgs copy = a;
+    void* args[] = {&copy};
+    ProfScope ps(name, st);
+    return cudaLaunchKernel((const void*)k, dim3((unsigned)g), dim3(128), args, 0, st);
+}
 cudaError_t spec_launch_prep(const PrepArgs& a, int prec, cudaStream_t st)
 {
     cudaKernel_t k;
@@ -533,14 +554,18 @@ cudaError_t spec_launch_prep(const PrepArgs& a, int prec, cudaStream_t st)
         if (!g_active) return cudaErrorNotReady;
         k = g_active->prep[prec == PREC_MIXED ? PREC_MIXED : PREC_FP64];
     }
-    int64_t n = (int64_t)(a.ghi[0] - a.glo[0] + 1) * (a.ghi[1] - a.glo[1] + 1) * (a.ghi[2] - a.glo[2] + 1);
-    int64_t g = (n + 127) / 128;
-    if (g > 148LL * 64) g = 148LL * 64;
-    if (g < 1) g = 1;
-    PrepArgs copy = a;
-    void* args[] = {&copy};
-    ProfScope ps("k_prep_spec", st);
-    return cudaLaunchKernel((const void*)k, dim3((unsigned)g), dim3(128), args, 0, st);
+    return launch_over(k, a, "k_prep_spec", st);
+}
+// the reaction source alone (a.glo..ghi the valid box), FP64
+cudaError_t spec_launch_source(const PrepArgs& a, cudaStream_t st)
+{
+    cudaKernel_t k;
+    {
+        std::lock_guard<std::mutex> lk(g_spec_mu);
+        if (!g_active) return cudaErrorNotReady;
+        k = g_active->source;
+    }
+    return launch_over(k, a, "k_reaction_source_spec", st);
 }
 
 // Batched form: boxes and items are device arrays; one CTA per work item (grid-stride).

@@ -32,10 +32,10 @@
 namespace vd {
 
 // ---------------------------------------------------------------------------
-// Joule heating at one cell (Source/ElecEnergySource.cpp:76-153).  USE_N: use the
-// per-cell density sums Nv (fused path) instead of re-summing the species.
-template <bool USE_N>
-__device__ __forceinline__ double joule_cell(const TransportArgs& a, int dim, int i, int j, int k)
+// Joule heating at one cell (Source/ElecEnergySource.cpp:76-153).  nsum(i, j, k): the
+// cell's density sum.
+template <class NSUM>
+__device__ __forceinline__ double joule_cell(const TransportArgs& a, int dim, int i, int j, int k, NSUM&& nsum)
 {
     const int ns = a.ns, eidx = a.e_id;
     double jheat = 0.0;
@@ -65,13 +65,7 @@ __device__ __forceinline__ double joule_cell(const TransportArgs& a, int dim, in
             double ne = 0.5 * (nel + ner);
             double ef = a.cs_technique ? evf_d : a.ef[idim](face[0], face[1], face[2]);
             double gn = a.gradne_from_state ? (ner - nel) / a.dx[idim] : a.gne[idim](face[0], face[1], face[2]);
-            double ndens;
-            if (USE_N) {
-                ndens = 0.5 * (a.Nv(l[0], l[1], l[2]) + a.Nv(face[0], face[1], face[2]));
-            } else {
-                ndens = 0.0;
-                for (int s = 0; s < ns; s++) ndens += 0.5 * (p[ol + s * cs] + p[orr + s * cs]);
-            }
+            const double ndens = 0.5 * (nsum(l[0], l[1], l[2]) + nsum(face[0], face[1], face[2]));
             double mu = a.const_ele_trans ? a.ele_mob / ndens : mob_fp64(eidx, etemp, ndens, a.Tg, emag);
             double dc = a.const_ele_trans ? a.ele_diff / ndens : diff_fp64(eidx, etemp, ndens, a.Tg, emag);
             double cur = a.charge_e * (mu * ne * ef - dc * gn);
