@@ -236,23 +236,35 @@ __global__ void __launch_bounds__(128) k_dif_residual(DLevel L, DBc bc, double* 
     }
 }
 
-// coarse rhs = average of the 2^dim fine residuals; coarse correction starts at 0
+// average of the 2^dim fine residuals under coarse cell (i,j,k), each formed here (no
+// residual array between the two levels)
 template <int DIM>
-__global__ void __launch_bounds__(128) k_dif_restrict(DLevel F, DLevel C)
+__device__ __forceinline__ double drestrict(const DLevel& F, const DBc& bc, int i, int j, int k)
 {
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= C.n[0]) return;
     double s = 0.0;
 #pragma unroll
     for (int dz = 0; dz < (DIM > 2 ? 2 : 1); dz++)
 #pragma unroll
         for (int dy = 0; dy < (DIM > 1 ? 2 : 1); dy++)
 #pragma unroll
-            for (int dx = 0; dx < 2; dx++)
-                s += F.res[dlin(F, 2 * i + dx, DIM > 1 ? 2 * j + dy : j, DIM > 2 ? 2 * k + dz : k)];
+            for (int dx = 0; dx < 2; dx++) {
+                const int fi = 2 * i + dx, fj = DIM > 1 ? 2 * j + dy : j, fk = DIM > 2 ? 2 * k + dz : k;
+                double off, diag;
+                dstencil<DIM>(F, bc, fi, fj, fk, F.phi, off, diag);
+                const int64_t c = dlin(F, fi, fj, fk);
+                s += F.rhs[c] - (off + diag * F.phi[c]);
+            }
+    return s * (1.0 / (double)(1 << DIM));
+}
+// coarse rhs = that average; coarse correction starts at 0
+template <int DIM>
+__global__ void __launch_bounds__(128) k_dif_restrict(DLevel F, DLevel C, DBc bc)
+{
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= C.n[0]) return;
     const int64_t c = dlin(C, i, j, k);
-    C.rhs[c] = s * (1.0 / (double)(1 << DIM));
+    C.rhs[c] = drestrict<DIM>(F, bc, i, j, k);
     C.phi[c] = 0.0;
 }
 
@@ -300,11 +312,8 @@ __global__ void __launch_bounds__(128) k_dif_coarsen_b(DLevel F, DLevel C)
 // relation for a Robin face, c otherwise; across a periodic direction the cell on
 // the other side
 template <int DIM>
-__global__ void __launch_bounds__(128) k_dif_prolong(DLevel F, DLevel C, DBc bc)
+__device__ __forceinline__ double dprolong(const DLevel& C, const DBc& bc, int i, int j, int k)
 {
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= F.n[0]) return;
     const int f[3] = {i, j, k};
     int ci[3] = {i, j, k}, nb[3] = {0, 0, 0};
 #pragma unroll
@@ -346,27 +355,162 @@ __global__ void __launch_bounds__(128) k_dif_prolong(DLevel F, DLevel C, DBc bc)
                 }
                 acc += w * sign * C.phi[dlin(C, q[0], q[1], q[2])];
             }
-    F.phi[dlin(F, i, j, k)] += acc;
+    return acc;
+}
+template <int DIM>
+__global__ void __launch_bounds__(128) k_dif_prolong(DLevel F, DLevel C, DBc bc)
+{
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= F.n[0]) return;
+    F.phi[dlin(F, i, j, k)] += dprolong<DIM>(C, bc, i, j, k);
 }
 
-constexpr int kDifBottomCells = 4096;
+// The coarse end of the V-cycle in one CTA: every level from the first whose arrays
+// fit shared memory (about 64^2 or 16^3 cells) down to the coarsest grid and back, with
+// a barrier between half sweeps.  The same operations on the same values as the
+// kernels above, one launch instead of eleven per level and a bottom solve; on
+// 512^2 these launches, 4 us each, were most of a cycle.  @@DC
+constexpr int kDifCoarseMax = 12;           // levels it may hold
+constexpr size_t kDifCoarseSmem = 220 * 1024;
+constexpr int kDifBottomSweeps = 64;
+struct DCoarse {
+    int nl;
+    int finest;  // its first level is the finest: inhomogeneous faces, starting values in phi
+    DLevel lv[kDifCoarseMax];
+    // 2^32 / n rounded up, for index divisions by n0, (n0 + 1) / 2 and n1
+    unsigned m0[kDifCoarseMax], mh[kDifCoarseMax], m1[kDifCoarseMax];
+};
+__host__ __device__ inline size_t dcoarse_doubles(const DLevel& L, int dim)
+{
+    size_t t = 2 * (size_t)L.cells();
+    for (int d = 0; d < dim; d++) t += (size_t)(L.n[0] + (d == 0)) * (L.n[1] + (d == 1)) * (L.n[2] + (d == 2));
+    return t;
+}
 
 template <int DIM>
-__global__ void __launch_bounds__(256) k_dif_bottom(DLevel L, DBc bc, int sweeps)
+__global__ void __launch_bounds__(512) k_dif_coarse(const __grid_constant__ DCoarse P, const __grid_constant__ DBc bcf,
+                                                     const __grid_constant__ DBc bc0)
 {
-    const int n0 = L.n[0], n1 = L.n[1];
-    const int nc = (int)L.cells();
-    for (int s = 0; s < sweeps; s++)
-        for (int color = 0; color < 2; color++) {
-            for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-                const int k = c / (n0 * n1), r = c - k * n0 * n1, j = r / n0, i = r - j * n0;
-                if (((i + j + k) & 1) != color) continue;
-                double off, diag;
-                dstencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
-                L.phi[c] = (L.rhs[c] - off) / diag;
+    extern __shared__ double sm[];
+    __shared__ DLevel lv[kDifCoarseMax];
+    const int tid = threadIdx.x, nth = blockDim.x;
+    {
+        double* p = sm;
+        for (int l = 0; l < P.nl; l++) {
+            const DLevel& G = P.lv[l];
+            const int nc = (int)G.cells();
+            double* phi = p;
+            double* rhs = p + nc;
+            p += 2 * nc;
+            for (int c = tid; c < nc; c += nth) {
+                phi[c] = (l == 0 && P.finest) ? G.phi[c] : 0.0;
+                if (l == 0) rhs[c] = G.rhs[c];
             }
+            double* b[3] = {nullptr, nullptr, nullptr};
+#pragma unroll
+            for (int d = 0; d < DIM; d++) {
+                b[d] = p;
+                const int nf = (G.n[0] + (d == 0)) * (G.n[1] + (d == 1)) * (G.n[2] + (d == 2));
+                for (int c = tid; c < nf; c += nth) p[c] = G.b[d][c];
+                p += nf;
+            }
+            if (tid == 0) {
+                DLevel L = G;
+                L.phi = phi;
+                L.rhs = rhs;
+                L.res = nullptr;
+                for (int d = 0; d < 3; d++) L.b[d] = b[d];
+                lv[l] = L;
+            }
+        }
+    }
+    __syncthreads();
+    // c / n, exact for the sizes here (c n < 2^32)
+    auto quot = [](int c, unsigned magic, int n) { return n == 1 ? c : (int)__umulhi((unsigned)c, magic); };
+    auto cell = [&](int l, int c, int& i, int& j, int& k) {
+        const int n0 = lv[l].n[0], n1 = lv[l].n[1];
+        const int row = DIM > 1 ? quot(c, P.m0[l], n0) : 0;
+        i = DIM > 1 ? c - row * n0 : c;
+        k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
+        j = DIM > 2 ? row - k * n1 : row;
+    };
+    // one half sweep by threads t, t + step, ... over the cells of a colour; whether
+    // a cell changed
+    auto half = [&](int l, int color, int t, int step) -> bool {
+        const DLevel& L = lv[l];
+        const DBc& bc = (l == 0 && P.finest) ? bcf : bc0;
+        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2, nq = h * n1 * L.n[2];
+        bool ch = false;
+        for (int q = t; q < nq; q += step) {
+            const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
+            const int k = DIM > 2 ? quot(row, P.m1[l], n1) : 0, j = DIM > 2 ? row - k * n1 : row;
+            const int i = 2 * (q - row * h) + ((j + k + color) & 1);
+            if (i >= n0) continue;
+            const int c = i + n0 * row;
+            double off, diag;
+            dstencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
+            const double v = (L.rhs[c] - off) / diag;
+            ch |= !(v == L.phi[c]);
+            L.phi[c] = v;
+        }
+        return ch;
+    };
+    for (int l = 0; l < P.nl - 1; l++) {
+        for (int s = 0; s < 4; s++) {
+            half(l, s & 1, tid, nth);
             __syncthreads();
         }
+        const DLevel& F = lv[l];
+        const DLevel& C = lv[l + 1];
+        const int nc = (int)C.cells();
+        for (int c = tid; c < nc; c += nth) {
+            int i, j, k;
+            cell(l + 1, c, i, j, k);
+            C.rhs[c] = drestrict<DIM>(F, (l == 0 && P.finest) ? bcf : bc0, i, j, k);
+        }
+        __syncthreads();
+    }
+    {
+        // the bottom solve ends early once a whole sweep changes nothing (every later
+        // one would repeat it)
+        const int l = P.nl - 1;
+        if ((int)lv[l].cells() <= 64) {
+            if (tid < 32) {
+                for (int s = 0; s < kDifBottomSweeps; s++) {
+                    bool ch = half(l, 0, tid, 32);
+                    __syncwarp();
+                    ch |= half(l, 1, tid, 32);
+                    __syncwarp();
+                    if (!__any_sync(0xffffffffu, ch)) break;
+                }
+            }
+            __syncthreads();
+        } else {
+            for (int s = 0; s < kDifBottomSweeps; s++) {
+                bool ch = half(l, 0, tid, nth);
+                __syncthreads();
+                ch |= half(l, 1, tid, nth);
+                if (!__syncthreads_or(ch)) break;
+            }
+        }
+    }
+    for (int l = P.nl - 2; l >= 0; l--) {
+        const DLevel& F = lv[l];
+        const int nc = (int)F.cells();
+        for (int c = tid; c < nc; c += nth) {
+            int i, j, k;
+            cell(l, c, i, j, k);
+            F.phi[c] += dprolong<DIM>(lv[l + 1], bc0, i, j, k);
+        }
+        __syncthreads();
+        for (int s = 0; s < 4; s++) {
+            half(l, s & 1, tid, nth);
+            __syncthreads();
+        }
+    }
+    const int nc = (int)lv[0].cells();
+    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
 }
 
 __global__ void k_dif_maxabs(const double* x, int64_t n, unsigned long long* out)
@@ -590,20 +734,29 @@ struct DifOps {
         ProfScope ps("k_dif_residual", st);
         k_dif_residual<DIM><<<dgrid(L), 128, 0, st>>>(L, b, mx);
     }
-    static void restrict_(const DLevel& F, const DLevel& C, cudaStream_t st)
+    static void restrict_(const DLevel& F, const DLevel& C, const DBc& b, cudaStream_t st)
     {
         ProfScope ps("k_dif_restrict", st);
-        k_dif_restrict<DIM><<<dgrid(C), 128, 0, st>>>(F, C);
+        k_dif_restrict<DIM><<<dgrid(C), 128, 0, st>>>(F, C, b);
     }
     static void prolong(const DLevel& F, const DLevel& C, const DBc& b, cudaStream_t st)
     {
         ProfScope ps("k_dif_prolong", st);
         k_dif_prolong<DIM><<<dgrid(F), 128, 0, st>>>(F, C, b);
     }
-    static void bottom(const DLevel& L, const DBc& b, int sweeps, cudaStream_t st)
+    static cudaError_t coarse(const DCoarse& P, const DBc& bf, const DBc& b0, cudaStream_t st)
     {
-        ProfScope ps("k_dif_bottom", st);
-        k_dif_bottom<DIM><<<1, 256, 0, st>>>(L, b, sweeps);
+        size_t bytes = 0;
+        for (int l = 0; l < P.nl; l++) bytes += dcoarse_doubles(P.lv[l], DIM) * sizeof(double);
+        cudaError_t e = cudaFuncSetAttribute(k_dif_coarse<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)kDifCoarseSmem);
+        if (e != cudaSuccess) return e;
+        // one or two cells of the first level's larger colour per thread
+        int64_t t = (P.lv[0].cells() + 1) / 2;
+        const unsigned nth = (unsigned)(t >= 512 ? 512 : (t + 31) / 32 * 32);
+        ProfScope ps("k_dif_coarse", st);
+        k_dif_coarse<DIM><<<1, nth, bytes, st>>>(P, bf, b0);
+        return cudaGetLastError();
     }
     static void coarsen_b(const DLevel& F, const DLevel& C, cudaStream_t st)
     {
@@ -646,9 +799,9 @@ struct DifOps {
 struct DifTable {
     void (*rbgs)(const DLevel&, const DBc&, int, cudaStream_t);
     void (*residual)(const DLevel&, const DBc&, double*, cudaStream_t);
-    void (*restrict_)(const DLevel&, const DLevel&, cudaStream_t);
+    void (*restrict_)(const DLevel&, const DLevel&, const DBc&, cudaStream_t);
     void (*prolong)(const DLevel&, const DLevel&, const DBc&, cudaStream_t);
-    void (*bottom)(const DLevel&, const DBc&, int, cudaStream_t);
+    cudaError_t (*coarse)(const DCoarse&, const DBc&, const DBc&, cudaStream_t);
     void (*coarsen_b)(const DLevel&, const DLevel&, cudaStream_t);
     void (*setup)(const DifArgs&, const DLevel&, double*, double* const*, double* const*, cudaStream_t);
 };
@@ -657,7 +810,7 @@ template <int DIM>
 DifTable dif_table()
 {
     return {DifOps<DIM>::rbgs,    DifOps<DIM>::residual,  DifOps<DIM>::restrict_, DifOps<DIM>::prolong,
-            DifOps<DIM>::bottom,  DifOps<DIM>::coarsen_b, DifOps<DIM>::setup};
+            DifOps<DIM>::coarse,  DifOps<DIM>::coarsen_b, DifOps<DIM>::setup};
 }
 
 }  // namespace
@@ -875,25 +1028,40 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
     for (size_t l = 1; l < lv.size(); l++) ops.coarsen_b(lv[l - 1], lv[l], st);
     if ((rc = fail_launch("solver set-up"))) return rc;
 
-    auto vcycle = [&]() {
-        const int nl = (int)lv.size();
-        for (int l = 0; l < nl; l++) {
-            const DBc& b = l == 0 ? bc : bc0;
-            if (l == nl - 1 && lv[l].cells() <= kDifBottomCells) {
-                ops.bottom(lv[l], b, 64, st);
-            } else {
-                const int sweeps = (l == nl - 1) ? 64 : 2;
-                for (int s = 0; s < sweeps; s++) {
-                    ops.rbgs(lv[l], b, 0, st);
-                    ops.rbgs(lv[l], b, 1, st);
-                }
-            }
-            if (l < nl - 1) {
-                ops.residual(lv[l], b, nullptr, st);
-                ops.restrict_(lv[l], lv[l + 1], st);
-            }
+    // the levels the coarse kernel takes: the last ones, as many as fit
+    const int nl = (int)lv.size();
+    int lc = nl;
+    {
+        size_t bytes = 0;
+        while (lc > 0 && nl - lc < kDifCoarseMax) {
+            bytes += dcoarse_doubles(lv[lc - 1], dim) * sizeof(double);
+            if (bytes > kDifCoarseSmem || lv[lc - 1].cells() > 32768) break;
+            lc--;
         }
-        for (int l = nl - 2; l >= 0; l--) {
+    }
+    DCoarse pc;
+    memset((void*)&pc, 0, sizeof(pc));
+    pc.nl = nl - lc;
+    pc.finest = lc == 0;
+    for (int l = lc; l < nl; l++) {
+        pc.lv[l - lc] = lv[l];
+        const auto magic = [](int n) { return (unsigned)((0x100000000ull + n - 1) / n); };
+        pc.m0[l - lc] = magic(lv[l].n[0]);
+        pc.mh[l - lc] = magic((lv[l].n[0] + 1) / 2);
+        pc.m1[l - lc] = magic(lv[l].n[1]);
+    }
+    auto vcycle = [&]() {
+        for (int l = 0; l < lc; l++) {
+            const DBc& b = l == 0 ? bc : bc0;
+            const int sweeps = (l == nl - 1) ? kDifBottomSweeps : 2;
+            for (int s = 0; s < sweeps; s++) {
+                ops.rbgs(lv[l], b, 0, st);
+                ops.rbgs(lv[l], b, 1, st);
+            }
+            if (l < nl - 1) ops.restrict_(lv[l], lv[l + 1], b, st);
+        }
+        if (lc < nl) ops.coarse(pc, bc, bc0, st);
+        for (int l = std::min(lc, nl - 1) - 1; l >= 0; l--) {
             const DBc& b = l == 0 ? bc : bc0;
             ops.prolong(lv[l], lv[l + 1], bc0, st);
             for (int s = 0; s < 2; s++) {

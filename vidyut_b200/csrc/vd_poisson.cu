@@ -169,18 +169,6 @@ __global__ void __launch_bounds__(128) k_mg_rbgs(CLevel L, BcInfo bc, int color,
     }
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(128) k_mg_residual(CLevel L, BcInfo bc)
-{
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= L.n[0]) return;
-    float off, diag;
-    stencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
-    const int64_t c = lin(L, i, j, k);
-    L.res[c] = L.rhs[c] - (off + diag * L.phi[c]);
-}
-
 // The defect of the FP64 potential P, r = rhs - L phi (FP64, inhomogeneous faces),
 // becomes the right-hand side of the finest correction level (times the scale of
 // its coefficients, rounded to FP32), whose correction starts at zero.
@@ -245,23 +233,35 @@ __global__ void __launch_bounds__(128) k_mg_correct(Level P, CLevel E)
     P.phi[c] += (double)E.phi[c];
 }
 
-// coarse rhs = average of the 2^dim fine residuals (full weighting for cell centres)
+// average of the 2^dim fine residuals under coarse cell (i,j,k) (full weighting for
+// cell centres), each formed here: no residual array between the two levels
 template <int DIM>
-__global__ void __launch_bounds__(128) k_mg_restrict(CLevel F, CLevel C)
+__device__ __forceinline__ float mg_restrict(const CLevel& F, const BcInfo& bc, int i, int j, int k)
 {
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= C.n[0]) return;
     float s = 0.0f;
 #pragma unroll
     for (int dz = 0; dz < (DIM > 2 ? 2 : 1); dz++)
 #pragma unroll
         for (int dy = 0; dy < (DIM > 1 ? 2 : 1); dy++)
 #pragma unroll
-            for (int dx = 0; dx < 2; dx++)
-                s += F.res[lin(F, 2 * i + dx, DIM > 1 ? 2 * j + dy : j, DIM > 2 ? 2 * k + dz : k)];
+            for (int dx = 0; dx < 2; dx++) {
+                const int fi = 2 * i + dx, fj = DIM > 1 ? 2 * j + dy : j, fk = DIM > 2 ? 2 * k + dz : k;
+                float off, diag;
+                stencil<DIM>(F, bc, fi, fj, fk, F.phi, off, diag);
+                const int64_t c = lin(F, fi, fj, fk);
+                s += F.rhs[c] - (off + diag * F.phi[c]);
+            }
+    return s * (1.0f / (float)(1 << DIM));
+}
+// coarse rhs = that average; coarse correction starts at 0
+template <int DIM>
+__global__ void __launch_bounds__(128) k_mg_restrict(CLevel F, CLevel C, BcInfo bc)
+{
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= C.n[0]) return;
     const int64_t c = lin(C, i, j, k);
-    C.rhs[c] = s * (1.0f / (float)(1 << DIM));
+    C.rhs[c] = mg_restrict<DIM>(F, bc, i, j, k);
     C.phi[c] = 0.0f;
 }
 
@@ -269,11 +269,8 @@ __global__ void __launch_bounds__(128) k_mg_restrict(CLevel F, CLevel C)
 // direction; at a domain face the outside coarse value is the correction's
 // boundary value: -c for a Dirichlet face (zero at the face), c for zero gradient)
 template <int DIM>
-__global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo bc)
+__device__ __forceinline__ float mg_prolong(const CLevel& C, const BcInfo& bc, int i, int j, int k)
 {
-    const int j = blockIdx.y, k = blockIdx.z;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= F.n[0]) return;
     const int f[3] = {i, j, k};
     // per direction the two coarse cells (as offsets) and their weights; beyond a
     // domain face the second is the parent itself, weighted -1/4 or 1/4; beyond dim
@@ -312,29 +309,141 @@ __global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo b
             const float v = w[0][0] * C.phi[row + off[0][0]] + w[0][1] * C.phi[row + off[0][1]];
             acc += (w[1][my] * w[2][mz]) * v;
         }
-    F.phi[lin(F, i, j, k)] += acc;
+    return acc;
+}
+template <int DIM>
+__global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo bc)
+{
+    const int j = blockIdx.y, k = blockIdx.z;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= F.n[0]) return;
+    F.phi[lin(F, i, j, k)] += mg_prolong<DIM>(C, bc, i, j, k);
 }
 
-// bottom solve of a small coarsest grid: one CTA runs every red-black sweep, with
-// a barrier between half sweeps (cells <= kBottomCells)
-constexpr int kBottomCells = 4096;
+// The coarse end of the V-cycle in one CTA: every level from the first whose arrays
+// fit shared memory (about 128^2 or 27^3 cells) down to the coarsest grid and back,
+// with a barrier between half sweeps: one launch instead of eleven per level and a
+// bottom solve.  @@MC
+constexpr int kCoarseMax = 12;  // levels it may hold
+constexpr int kCoarseCells = 27000;  // cells of all of them (two floats each, 216 KB)
+constexpr int kBottomSweeps = 64;
+struct MCoarse {
+    int nl;
+    CLevel lv[kCoarseMax];
+    // 2^32 / n rounded up, for index divisions by n0, (n0 + 1) / 2 and n1
+    unsigned m0[kCoarseMax], mh[kCoarseMax], m1[kCoarseMax];
+};
 
 template <int DIM>
-__global__ void __launch_bounds__(256) k_mg_bottom(CLevel L, BcInfo bc, int sweeps)
+__global__ void __launch_bounds__(1024) k_mg_coarse(const __grid_constant__ MCoarse P, const __grid_constant__ BcInfo bc)
 {
-    const int n0 = L.n[0], n1 = L.n[1];
-    const int nc = (int)L.cells();
-    for (int s = 0; s < sweeps; s++)
-        for (int color = 0; color < 2; color++) {
-            for (int c = threadIdx.x; c < nc; c += blockDim.x) {
-                const int k = c / (n0 * n1), r = c - k * n0 * n1, j = r / n0, i = r - j * n0;
-                if (((i + j + k) & 1) != color) continue;
-                float off, diag;
-                stencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
-                L.phi[c] = __fdividef(L.rhs[c] - off, diag);
+    extern __shared__ float smf[];
+    __shared__ CLevel lv[kCoarseMax];
+    const int tid = threadIdx.x, nth = blockDim.x;
+    {
+        float* p = smf;
+        for (int l = 0; l < P.nl; l++) {
+            const CLevel& G = P.lv[l];
+            const int nc = (int)G.cells();
+            float* phi = p;
+            float* rhs = p + nc;
+            p += 2 * nc;
+            for (int c = tid; c < nc; c += nth) {
+                phi[c] = 0.0f;
+                if (l == 0) rhs[c] = G.rhs[c];
             }
+            if (tid == 0) {
+                CLevel L = G;
+                L.phi = phi;
+                L.rhs = rhs;
+                L.res = nullptr;
+                lv[l] = L;
+            }
+        }
+    }
+    __syncthreads();
+    // c / n, exact for the sizes here (c n < 2^32)
+    auto quot = [](int c, unsigned magic, int n) { return n == 1 ? c : (int)__umulhi((unsigned)c, magic); };
+    auto cell = [&](int l, int c, int& i, int& j, int& k) {
+        const int n0 = lv[l].n[0], n1 = lv[l].n[1];
+        const int row = DIM > 1 ? quot(c, P.m0[l], n0) : 0;
+        i = DIM > 1 ? c - row * n0 : c;
+        k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
+        j = DIM > 2 ? row - k * n1 : row;
+    };
+    // one half sweep by threads t, t + step, ... over the cells of a colour; whether
+    // a cell changed
+    auto half = [&](int l, int color, int t, int step) -> bool {
+        const CLevel& L = lv[l];
+        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2, nq = h * n1 * L.n[2];
+        bool ch = false;
+        for (int q = t; q < nq; q += step) {
+            const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
+            const int k = DIM > 2 ? quot(row, P.m1[l], n1) : 0, j = DIM > 2 ? row - k * n1 : row;
+            const int i = 2 * (q - row * h) + ((j + k + color) & 1);
+            if (i >= n0) continue;
+            const int c = i + n0 * row;
+            float off, diag;
+            stencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
+            const float v = __fdividef(L.rhs[c] - off, diag);
+            ch |= !(v == L.phi[c]);
+            L.phi[c] = v;
+        }
+        return ch;
+    };
+    for (int l = 0; l < P.nl - 1; l++) {
+        for (int s = 0; s < 4; s++) {
+            half(l, s & 1, tid, nth);
             __syncthreads();
         }
+        const CLevel& C = lv[l + 1];
+        const int nc = (int)C.cells();
+        for (int c = tid; c < nc; c += nth) {
+            int i, j, k;
+            cell(l + 1, c, i, j, k);
+            C.rhs[c] = mg_restrict<DIM>(lv[l], bc, i, j, k);
+        }
+        __syncthreads();
+    }
+    {
+        // ends early once a whole sweep changes nothing (every later one would repeat it)
+        const int l = P.nl - 1;
+        if ((int)lv[l].cells() <= 64) {
+            if (tid < 32) {
+                for (int s = 0; s < kBottomSweeps; s++) {
+                    bool ch = half(l, 0, tid, 32);
+                    __syncwarp();
+                    ch |= half(l, 1, tid, 32);
+                    __syncwarp();
+                    if (!__any_sync(0xffffffffu, ch)) break;
+                }
+            }
+            __syncthreads();
+        } else {
+            for (int s = 0; s < kBottomSweeps; s++) {
+                bool ch = half(l, 0, tid, nth);
+                __syncthreads();
+                ch |= half(l, 1, tid, nth);
+                if (!__syncthreads_or(ch)) break;
+            }
+        }
+    }
+    for (int l = P.nl - 2; l >= 0; l--) {
+        const CLevel& F = lv[l];
+        const int nc = (int)F.cells();
+        for (int c = tid; c < nc; c += nth) {
+            int i, j, k;
+            cell(l, c, i, j, k);
+            F.phi[c] += mg_prolong<DIM>(lv[l + 1], bc, i, j, k);
+        }
+        __syncthreads();
+        for (int s = 0; s < 4; s++) {
+            half(l, s & 1, tid, nth);
+            __syncthreads();
+        }
+    }
+    const int nc = (int)lv[0].cells();
+    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
 }
 
 template <class T>
@@ -366,20 +475,23 @@ struct Mg {
         const dim3 g = grid_pairs(L, DIM, 2, &half);
         k_mg_rbgs<DIM><<<g, 128, 0, st>>>(L, b, color, half, corr);
     }
-    static void residual(const CLevel& L, const BcInfo& b, cudaStream_t st)
-    {
-        ProfScope ps("k_mg_residual", st);
-        k_mg_residual<DIM><<<grid_cells(L), 128, 0, st>>>(L, b);
-    }
-    static void restrict_(const CLevel& F, const CLevel& C, cudaStream_t st)
+    static void restrict_(const CLevel& F, const CLevel& C, const BcInfo& b, cudaStream_t st)
     {
         ProfScope ps("k_mg_restrict", st);
-        k_mg_restrict<DIM><<<grid_cells(C), 128, 0, st>>>(F, C);
+        k_mg_restrict<DIM><<<grid_cells(C), 128, 0, st>>>(F, C, b);
     }
-    static void bottom(const CLevel& L, const BcInfo& b, int sweeps, cudaStream_t st)
+    static cudaError_t coarse(const MCoarse& P, const BcInfo& b, cudaStream_t st)
     {
-        ProfScope ps("k_mg_bottom", st);
-        k_mg_bottom<DIM><<<1, 256, 0, st>>>(L, b, sweeps);
+        size_t cells = 0;
+        for (int l = 0; l < P.nl; l++) cells += (size_t)P.lv[l].cells();
+        cudaError_t e = cudaFuncSetAttribute(k_mg_coarse<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             kCoarseCells * 2 * (int)sizeof(float));
+        if (e != cudaSuccess) return e;
+        int64_t t = (P.lv[0].cells() + 1) / 2;
+        const unsigned nth = (unsigned)(t >= 1024 ? 1024 : (t + 31) / 32 * 32);
+        ProfScope ps("k_mg_coarse", st);
+        k_mg_coarse<DIM><<<1, nth, 2 * cells * sizeof(float), st>>>(P, b);
+        return cudaGetLastError();
     }
     static void prolong(const CLevel& F, const CLevel& C, const BcInfo& b, cudaStream_t st)
     {
@@ -398,19 +510,18 @@ struct Mg {
 
 struct MgOps {
     void (*rbgs)(const CLevel&, const BcInfo&, int, double*, cudaStream_t);
-    void (*residual)(const CLevel&, const BcInfo&, cudaStream_t);
-    void (*restrict_)(const CLevel&, const CLevel&, cudaStream_t);
+    void (*restrict_)(const CLevel&, const CLevel&, const BcInfo&, cudaStream_t);
     void (*prolong)(const CLevel&, const CLevel&, const BcInfo&, cudaStream_t);
-    void (*bottom)(const CLevel&, const BcInfo&, int, cudaStream_t);
+    cudaError_t (*coarse)(const MCoarse&, const BcInfo&, cudaStream_t);
     void (*defect)(const Level&, const BcInfo&, const CLevel&, double, double*, cudaStream_t);
 };
 
-MgOps mg_ops(int dim)
+template <int DIM>
+MgOps mg_ops_of()
 {
-    if (dim == 1) return {Mg<1>::rbgs, Mg<1>::residual, Mg<1>::restrict_, Mg<1>::prolong, Mg<1>::bottom, Mg<1>::defect};
-    if (dim == 2) return {Mg<2>::rbgs, Mg<2>::residual, Mg<2>::restrict_, Mg<2>::prolong, Mg<2>::bottom, Mg<2>::defect};
-    return {Mg<3>::rbgs, Mg<3>::residual, Mg<3>::restrict_, Mg<3>::prolong, Mg<3>::bottom, Mg<3>::defect};
+    return {Mg<DIM>::rbgs, Mg<DIM>::restrict_, Mg<DIM>::prolong, Mg<DIM>::coarse, Mg<DIM>::defect};
 }
+MgOps mg_ops(int dim) { return dim == 1 ? mg_ops_of<1>() : dim == 2 ? mg_ops_of<2>() : mg_ops_of<3>(); }
 
 __global__ void k_maxabs(const double* x, int64_t n, unsigned long long* out)
 {
@@ -703,31 +814,46 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
     const MgOps ops = mg_ops(dim);
     // one V(2,2) cycle of the correction equation, from a zero correction, then the
     // correction added to the potential (inside the last half sweep)
-    auto vcycle = [&]() {
-        const int nl = (int)lv.size();
-        for (int l = 0; l < nl; l++) {
-            if (l == nl - 1 && lv[l].cells() <= kBottomCells) {
-                ops.bottom(lv[l], bc0, 64, st);  // one CTA, all sweeps in one launch
-            } else {
-                const int sweeps = (l == nl - 1) ? 64 : 2;
-                for (int s = 0; s < sweeps; s++) {
-                    ops.rbgs(lv[l], bc0, 0, nullptr, st);
-                    ops.rbgs(lv[l], bc0, 1, nullptr, st);
-                }
-            }
-            if (l < nl - 1) {
-                ops.residual(lv[l], bc0, st);
-                ops.restrict_(lv[l], lv[l + 1], st);
-            }
+    // the levels the coarse kernel takes: the last ones, as many as fit
+    const int nl = (int)lv.size();
+    int lc = nl;
+    {
+        int64_t cells = 0;
+        while (lc > 0 && nl - lc < kCoarseMax) {
+            cells += lv[lc - 1].cells();
+            if (cells > kCoarseCells) break;
+            lc--;
         }
-        for (int l = nl - 2; l >= 0; l--) {
+    }
+    MCoarse pc;
+    memset((void*)&pc, 0, sizeof(pc));
+    pc.nl = nl - lc;
+    for (int l = lc; l < nl; l++) {
+        pc.lv[l - lc] = lv[l];
+        const auto magic = [](int n) { return (unsigned)((0x100000000ull + n - 1) / n); };
+        pc.m0[l - lc] = magic(lv[l].n[0]);
+        pc.mh[l - lc] = magic((lv[l].n[0] + 1) / 2);
+        pc.m1[l - lc] = magic(lv[l].n[1]);
+    }
+    auto vcycle = [&]() {
+        for (int l = 0; l < lc; l++) {
+            const int sweeps = (l == nl - 1) ? kBottomSweeps : 2;
+            for (int s = 0; s < sweeps; s++) {
+                ops.rbgs(lv[l], bc0, 0, nullptr, st);
+                ops.rbgs(lv[l], bc0, 1, nullptr, st);
+            }
+            if (l < nl - 1) ops.restrict_(lv[l], lv[l + 1], bc0, st);
+        }
+        if (lc < nl) ops.coarse(pc, bc0, st);
+        const bool fine = lc > 0 && nl > 1;  // the finest level is smoothed by its own launches
+        for (int l = std::min(lc, nl - 1) - 1; l >= 0; l--) {
             ops.prolong(lv[l], lv[l + 1], bc0, st);
             for (int s = 0; s < 2; s++) {
                 ops.rbgs(lv[l], bc0, 0, nullptr, st);
                 ops.rbgs(lv[l], bc0, 1, (l == 0 && s == 1) ? P.phi : nullptr, st);
             }
         }
-        if (nl == 1) {  // no coarser level: the cycle was the bottom solve
+        if (!fine) {  // the whole cycle was one launch, or the bottom solve
             ProfScope ps("k_mg_correct", st);
             k_mg_correct<<<grid_cells(P), 128, 0, st>>>(P, lv[0]);
         }
