@@ -31,6 +31,7 @@
 #include <vector>
 #include "vd_device.cuh"
 #include "vd_host.h"
+#include "vd_mg2d.cuh"
 
 namespace vd {
 
@@ -512,6 +513,26 @@ __global__ void __launch_bounds__(512) k_dif_coarse(const __grid_constant__ DCoa
     const int nc = (int)lv[0].cells();
     for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
 }
+
+// the operator of a 2-D level as the fused legs take it (vd_mg2d.cuh)
+struct DOp2 {
+    using T = double;
+    static constexpr int kCoef = 2;
+    int n[2];
+    DLevel L, C;  // C: the next coarser level
+    DBc bc, bcc;  // faces of L, and the homogeneous ones of the prolongation
+    __device__ __forceinline__ double rhs(int64_t c) const { return L.rhs[c]; }
+    __device__ __forceinline__ double coef(int d, int i, int j) const { return L.b[d][flin(L, d, i, j, 0)]; }
+    __device__ __forceinline__ void row(int i, int j, double x0, double x1, double y0, double y1, double bx0,
+                                        double bx1, double by0, double by1, double& off, double& diag) const
+    {
+        const DNbr<2> v{{bx0, by0}, {bx1, by1}, {x0, y0}, {x1, y1}};
+        dstencil_apply<2>(L, bc, i, j, 0, v, off, diag);
+    }
+    __device__ __forceinline__ double quot(double a, double b) const { return a / b; }
+    __device__ __forceinline__ double prolong(int i, int j) const { return dprolong<2>(C, bcc, i, j, 0); }
+    __device__ __forceinline__ void restrict_to(int i, int j, double r) const { C.rhs[dlin(C, i, j, 0)] = r; }
+};
 
 __global__ void k_dif_maxabs(const double* x, int64_t n, unsigned long long* out)
 {
@@ -1050,9 +1071,32 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         pc.mh[l - lc] = magic((lv[l].n[0] + 1) / 2);
         pc.m1[l - lc] = magic(lv[l].n[1]);
     }
-    auto vcycle = [&]() {
+    // 2-D levels with a coarser one take each leg of the cycle in one kernel, whose
+    // result goes to the level's other array (res) and back; a periodic direction
+    // keeps the separate kernels (the tiles do not wrap)
+    const bool legs = dim == 2 && !bc.per[0] && !bc.per[1];
+    auto leg = [&](int l, bool up, unsigned long long* mx) {
+        DOp2 op;
+        op.n[0] = lv[l].n[0];
+        op.n[1] = lv[l].n[1];
+        op.L = lv[l];
+        op.C = lv[l + 1];
+        op.bc = l == 0 ? bc : bc0;
+        op.bcc = bc0;
+        ProfScope ps(up ? "k_dif_leg_up" : "k_dif_leg_down", st);
+        const dim3 g = mg2d_grid(op.n);
+        if (up) k_mg2d<DOp2, true><<<g, kMg2Threads, 0, st>>>(op, lv[l].res, lv[l].phi, nullptr, mx);
+        else k_mg2d<DOp2, false><<<g, kMg2Threads, 0, st>>>(op, l == 0 ? lv[l].phi : nullptr, lv[l].res, nullptr, nullptr);
+    };
+    const bool leg0 = legs && lc > 0 && nl > 1;  // the finest level goes by legs
+    // mx (leg0 only): the residual's maximum, formed by the last leg
+    auto vcycle = [&](unsigned long long* mx) {
         for (int l = 0; l < lc; l++) {
             const DBc& b = l == 0 ? bc : bc0;
+            if (legs && l < nl - 1) {
+                leg(l, false, nullptr);
+                continue;
+            }
             const int sweeps = (l == nl - 1) ? kDifBottomSweeps : 2;
             for (int s = 0; s < sweeps; s++) {
                 ops.rbgs(lv[l], b, 0, st);
@@ -1063,6 +1107,10 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         if (lc < nl) ops.coarse(pc, bc, bc0, st);
         for (int l = std::min(lc, nl - 1) - 1; l >= 0; l--) {
             const DBc& b = l == 0 ? bc : bc0;
+            if (legs) {
+                leg(l, true, l == 0 ? mx : nullptr);
+                continue;
+            }
             ops.prolong(lv[l], lv[l + 1], bc0, st);
             for (int s = 0; s < 2; s++) {
                 ops.rbgs(lv[l], b, 0, st);
@@ -1071,8 +1119,10 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         }
     };
     auto maxabs = [&](bool resid, double* out) -> int {
-        cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st);
-        if (resid) {
+        if (!(resid && leg0)) cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st);
+        if (resid && leg0) {
+            // the last leg left it in d_max
+        } else if (resid) {
             ops.residual(lv[0], bc, blkmax, st);
             ProfScope ps("k_dif_maxabs", st);
             const unsigned g = (unsigned)std::min<int64_t>((nblk0 + 255) / 256, 148 * 32);
@@ -1100,7 +1150,8 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         }
         if (scale == 0.0) scale = 1.0;
         for (done = 0; done < dp->max_vcycles;) {
-            vcycle();
+            if (leg0) cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st);
+            vcycle(leg0 ? d_max : nullptr);
             done++;
             if ((rc = maxabs(true, &r))) {
                 cudaFreeAsync(buf, st);
@@ -1114,7 +1165,7 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
             return derr(VD_ERR_CUDA, "the species solve produced a non-finite residual");
         }
     } else {
-        for (done = 0; done < dp->max_vcycles; done++) vcycle();
+        for (done = 0; done < dp->max_vcycles; done++) vcycle(nullptr);
     }
     {
         ProfScope ps("k_dif_finish", st);

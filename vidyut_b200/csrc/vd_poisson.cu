@@ -21,6 +21,7 @@
 #include <cstring>
 #include <vector>
 #include "vd_host.h"
+#include "vd_mg2d.cuh"
 
 namespace vd {
 namespace {
@@ -446,6 +447,26 @@ __global__ void __launch_bounds__(1024) k_mg_coarse(const __grid_constant__ MCoa
     for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
 }
 
+// the operator of a 2-D correction level as the fused legs take it (vd_mg2d.cuh)
+struct MOp2 {
+    using T = float;
+    static constexpr int kCoef = 0;
+    int n[2];
+    CLevel L, C;  // C: the next coarser level
+    BcInfo bc;
+    __device__ __forceinline__ float rhs(int64_t c) const { return L.rhs[c]; }
+    __device__ __forceinline__ float coef(int, int, int) const { return 0.0f; }
+    __device__ __forceinline__ void row(int i, int j, float x0, float x1, float y0, float y1, float& off,
+                                        float& diag) const
+    {
+        const Nbr<2, float> v{{x0, y0}, {x1, y1}};
+        stencil_apply<2>(L, bc, i, j, 0, v, off, diag);
+    }
+    __device__ __forceinline__ float quot(float a, float b) const { return __fdividef(a, b); }
+    __device__ __forceinline__ float prolong(int i, int j) const { return mg_prolong<2>(C, bc, i, j, 0); }
+    __device__ __forceinline__ void restrict_to(int i, int j, float r) const { C.rhs[lin(C, i, j, 0)] = r; }
+};
+
 template <class T>
 dim3 grid_cells(const LevelT<T>& L, int per_thread = 1)
 {
@@ -835,8 +856,26 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         pc.mh[l - lc] = magic((lv[l].n[0] + 1) / 2);
         pc.m1[l - lc] = magic(lv[l].n[1]);
     }
+    // 2-D levels with a coarser one take each leg of the cycle in one kernel, whose
+    // result goes to the level's other array (res) and back
+    auto leg = [&](int l, bool up) {
+        MOp2 op;
+        op.n[0] = lv[l].n[0];
+        op.n[1] = lv[l].n[1];
+        op.L = lv[l];
+        op.C = lv[l + 1];
+        op.bc = bc0;
+        ProfScope ps(up ? "k_mg_leg_up" : "k_mg_leg_down", st);
+        const dim3 g = mg2d_grid(op.n);
+        if (up) k_mg2d<MOp2, true><<<g, kMg2Threads, 0, st>>>(op, lv[l].res, lv[l].phi, l == 0 ? P.phi : nullptr, nullptr);
+        else k_mg2d<MOp2, false><<<g, kMg2Threads, 0, st>>>(op, nullptr, lv[l].res, nullptr, nullptr);
+    };
     auto vcycle = [&]() {
         for (int l = 0; l < lc; l++) {
+            if (dim == 2 && l < nl - 1) {
+                leg(l, false);
+                continue;
+            }
             const int sweeps = (l == nl - 1) ? kBottomSweeps : 2;
             for (int s = 0; s < sweeps; s++) {
                 ops.rbgs(lv[l], bc0, 0, nullptr, st);
@@ -847,6 +886,10 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         if (lc < nl) ops.coarse(pc, bc0, st);
         const bool fine = lc > 0 && nl > 1;  // the finest level is smoothed by its own launches
         for (int l = std::min(lc, nl - 1) - 1; l >= 0; l--) {
+            if (dim == 2) {
+                leg(l, true);
+                continue;
+            }
             ops.prolong(lv[l], lv[l + 1], bc0, st);
             for (int s = 0; s < 2; s++) {
                 ops.rbgs(lv[l], bc0, 0, nullptr, st);
