@@ -371,10 +371,12 @@ __global__ void __launch_bounds__(128) k_dif_prolong(DLevel F, DLevel C, DBc bc)
 // fit shared memory (about 64^2 or 16^3 cells) down to the coarsest grid and back, with
 // a barrier between half sweeps.  The same operations on the same values as the
 // kernels above, one launch instead of eleven per level and a bottom solve; on
-// 512^2 these launches, 4 us each, were most of a cycle.  @@DC
+// 512^2 these launches, 4 us each, were most of a cycle (electron solve 2.15 ms; 0.80 ms
+// with this and the legs below).
 constexpr int kDifCoarseMax = 12;           // levels it may hold
 constexpr size_t kDifCoarseSmem = 220 * 1024;
 constexpr int kDifBottomSweeps = 64;
+constexpr int64_t kDifCoarse2 = 1100;  // 2-D: larger levels go by legs (512^2 826 us; 4096: 880 us)
 struct DCoarse {
     int nl;
     int finest;  // its first level is the finest: inhomogeneous faces, starting values in phi
@@ -394,124 +396,163 @@ __global__ void __launch_bounds__(512) k_dif_coarse(const __grid_constant__ DCoa
                                                      const __grid_constant__ DBc bc0)
 {
     extern __shared__ double sm[];
-    __shared__ DLevel lv[kDifCoarseMax];
+    __shared__ int soff[kDifCoarseMax + 1];  // where each level's arrays begin
     const int tid = threadIdx.x, nth = blockDim.x;
+    auto level = [&](int l) {
+        DLevel L = P.lv[l];
+        const int nc = (int)L.cells();
+        L.phi = sm + soff[l];
+        L.rhs = L.phi + nc;
+        L.res = nullptr;
+        double* p = L.rhs + nc;
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            L.b[d] = p;
+            p += (L.n[0] + (d == 0)) * (L.n[1] + (d == 1)) * (L.n[2] + (d == 2));
+        }
+        return L;
+    };
     {
-        double* p = sm;
+        int o = 0;
         for (int l = 0; l < P.nl; l++) {
             const DLevel& G = P.lv[l];
             const int nc = (int)G.cells();
-            double* phi = p;
-            double* rhs = p + nc;
-            p += 2 * nc;
+            if (tid == 0) soff[l] = o;
             for (int c = tid; c < nc; c += nth) {
-                phi[c] = (l == 0 && P.finest) ? G.phi[c] : 0.0;
-                if (l == 0) rhs[c] = G.rhs[c];
+                sm[o + c] = (l == 0 && P.finest) ? G.phi[c] : 0.0;
+                if (l == 0) sm[o + nc + c] = G.rhs[c];
             }
-            double* b[3] = {nullptr, nullptr, nullptr};
+            o += 2 * nc;
 #pragma unroll
             for (int d = 0; d < DIM; d++) {
-                b[d] = p;
                 const int nf = (G.n[0] + (d == 0)) * (G.n[1] + (d == 1)) * (G.n[2] + (d == 2));
-                for (int c = tid; c < nf; c += nth) p[c] = G.b[d][c];
-                p += nf;
-            }
-            if (tid == 0) {
-                DLevel L = G;
-                L.phi = phi;
-                L.rhs = rhs;
-                L.res = nullptr;
-                for (int d = 0; d < 3; d++) L.b[d] = b[d];
-                lv[l] = L;
+                for (int c = tid; c < nf; c += nth) sm[o + c] = G.b[d][c];
+                o += nf;
             }
         }
     }
     __syncthreads();
     // c / n, exact for the sizes here (c n < 2^32)
     auto quot = [](int c, unsigned magic, int n) { return n == 1 ? c : (int)__umulhi((unsigned)c, magic); };
-    auto cell = [&](int l, int c, int& i, int& j, int& k) {
-        const int n0 = lv[l].n[0], n1 = lv[l].n[1];
+    auto cell = [&](const DLevel& L, int l, int c, int& i, int& j, int& k) {
+        const int n0 = L.n[0], n1 = L.n[1];
         const int row = DIM > 1 ? quot(c, P.m0[l], n0) : 0;
         i = DIM > 1 ? c - row * n0 : c;
         k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
         j = DIM > 2 ? row - k * n1 : row;
     };
-    // one half sweep by threads t, t + step, ... over the cells of a colour; whether
-    // a cell changed
-    auto half = [&](int l, int color, int t, int step) -> bool {
-        const DLevel& L = lv[l];
-        const DBc& bc = (l == 0 && P.finest) ? bcf : bc0;
-        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2, nq = h * n1 * L.n[2];
-        bool ch = false;
-        for (int q = t; q < nq; q += step) {
-            const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
-            const int k = DIM > 2 ? quot(row, P.m1[l], n1) : 0, j = DIM > 2 ? row - k * n1 : row;
-            const int i = 2 * (q - row * h) + ((j + k + color) & 1);
-            if (i >= n0) continue;
-            const int c = i + n0 * row;
-            double off, diag;
-            dstencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
-            const double v = (L.rhs[c] - off) / diag;
-            ch |= !(v == L.phi[c]);
-            L.phi[c] = v;
-        }
-        return ch;
+    // cell q of a colour: x pair fastest, then the rows; false past the row's end
+    auto colour_cell = [&](const DLevel& L, int l, int color, int q, int& i, int& j, int& k, int& c) {
+        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2;
+        const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
+        k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
+        j = DIM > 2 ? row - k * n1 : row;
+        i = 2 * (q - row * h) + ((j + k + color) & 1);
+        c = i + n0 * row;
+        return i < n0;
     };
-    for (int l = 0; l < P.nl - 1; l++) {
+    auto sweeps2 = [&](const DLevel& L, int l) {
+        const DBc& bc = (l == 0 && P.finest) ? bcf : bc0;
+        const int nq = (L.n[0] + 1) / 2 * L.n[1] * L.n[2];
         for (int s = 0; s < 4; s++) {
-            half(l, s & 1, tid, nth);
+            for (int q = tid; q < nq; q += nth) {
+                int i, j, k, c;
+                if (!colour_cell(L, l, s & 1, q, i, j, k, c)) continue;
+                double off, diag;
+                dstencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
+                L.phi[c] = (L.rhs[c] - off) / diag;
+            }
             __syncthreads();
         }
-        const DLevel& F = lv[l];
-        const DLevel& C = lv[l + 1];
+    };
+    for (int l = 0; l < P.nl - 1; l++) {
+        const DLevel F = level(l), C = level(l + 1);
+        sweeps2(F, l);
         const int nc = (int)C.cells();
         for (int c = tid; c < nc; c += nth) {
             int i, j, k;
-            cell(l + 1, c, i, j, k);
+            cell(C, l + 1, c, i, j, k);
             C.rhs[c] = drestrict<DIM>(F, (l == 0 && P.finest) ? bcf : bc0, i, j, k);
         }
         __syncthreads();
     }
     {
-        // the bottom solve ends early once a whole sweep changes nothing (every later
-        // one would repeat it)
+        // Bottom solve.  Up to one cell of each colour per thread: its neighbours' places,
+        // their coefficients (0 beyond a domain face, whose value is 0 on a correction
+        // level), the diagonal and the right-hand side stay in registers, and only the
+        // warps that hold cells take part (one warp: no barrier, and it ends once a
+        // whole sweep changes nothing, as every later one would repeat it).
         const int l = P.nl - 1;
-        if ((int)lv[l].cells() <= 64) {
-            if (tid < 32) {
+        const DLevel L = level(l);
+        const int nq = (L.n[0] + 1) / 2 * L.n[1] * L.n[2];
+        if (nq <= nth && (P.nl > 1 || !P.finest)) {
+            const int nb = (nq + 31) / 32 * 32;
+            if (tid < nb) {
+                double* at[2];
+                int lo[2][DIM], hi[2][DIM];
+                double wl[2][DIM], wh[2][DIM], diag[2], r[2];
+                bool ok[2];
+#pragma unroll
+                for (int color = 0; color < 2; color++) {
+                    int i, j, k, c;
+                    ok[color] = colour_cell(L, l, color, tid, i, j, k, c) && tid < nq;
+                    if (!ok[color]) continue;
+                    at[color] = L.phi + c;
+                    r[color] = L.rhs[c];
+                    double off;
+                    const DNbr<DIM> nb1 = dstencil_load<DIM>(L, bc0, i, j, k, L.phi);
+                    dstencil_apply<DIM>(L, bc0, i, j, k, nb1, off, diag[color]);
+                    const int cc[3] = {i, j, k}, str[3] = {1, L.n[0], L.n[0] * L.n[1]};
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) {
+                        const int n = L.n[d];
+                        const bool l1 = cc[d] > 0 || bc0.per[d], h1 = cc[d] < n - 1 || bc0.per[d];
+                        lo[color][d] = cc[d] > 0 ? -str[d] : (l1 ? (n - 1) * str[d] : 0);
+                        hi[color][d] = cc[d] < n - 1 ? str[d] : (h1 ? -(n - 1) * str[d] : 0);
+                        wl[color][d] = l1 ? -(nb1.blo[d] * L.idx2[d]) : 0.0;
+                        wh[color][d] = h1 ? -(nb1.bhi[d] * L.idx2[d]) : 0.0;
+                    }
+                }
                 for (int s = 0; s < kDifBottomSweeps; s++) {
-                    bool ch = half(l, 0, tid, 32);
-                    __syncwarp();
-                    ch |= half(l, 1, tid, 32);
-                    __syncwarp();
-                    if (!__any_sync(0xffffffffu, ch)) break;
+                    bool ch = false;
+#pragma unroll
+                    for (int color = 0; color < 2; color++) {
+                        if (ok[color]) {
+                            double off = 0;
+#pragma unroll
+                            for (int d = 0; d < DIM; d++) {
+                                off = fma(wl[color][d], at[color][lo[color][d]], off);
+                                off = fma(wh[color][d], at[color][hi[color][d]], off);
+                            }
+                            const double v = (r[color] - off) / diag[color];
+                            ch |= !(v == *at[color]);
+                            *at[color] = v;
+                        }
+                        if (nb == 32) __syncwarp();
+                        else asm volatile("bar.sync 1, %0;" ::"r"(nb) : "memory");
+                    }
+                    if (nb == 32 && !__any_sync(0xffffffffu, ch)) break;
                 }
             }
             __syncthreads();
         } else {
-            for (int s = 0; s < kDifBottomSweeps; s++) {
-                bool ch = half(l, 0, tid, nth);
-                __syncthreads();
-                ch |= half(l, 1, tid, nth);
-                if (!__syncthreads_or(ch)) break;
-            }
+            for (int s = 0; s < kDifBottomSweeps / 2; s++) sweeps2(L, l);
         }
     }
     for (int l = P.nl - 2; l >= 0; l--) {
-        const DLevel& F = lv[l];
+        const DLevel F = level(l), C = level(l + 1);
         const int nc = (int)F.cells();
         for (int c = tid; c < nc; c += nth) {
             int i, j, k;
-            cell(l, c, i, j, k);
-            F.phi[c] += dprolong<DIM>(lv[l + 1], bc0, i, j, k);
+            cell(F, l, c, i, j, k);
+            F.phi[c] += dprolong<DIM>(C, bc0, i, j, k);
         }
         __syncthreads();
-        for (int s = 0; s < 4; s++) {
-            half(l, s & 1, tid, nth);
-            __syncthreads();
-        }
+        sweeps2(F, l);
     }
-    const int nc = (int)lv[0].cells();
-    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
+    const DLevel L0 = level(0);
+    const int nc = (int)L0.cells();
+    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = L0.phi[c];
 }
 
 // the operator of a 2-D level as the fused legs take it (vd_mg2d.cuh)
@@ -773,7 +814,7 @@ struct DifOps {
                                              (int)kDifCoarseSmem);
         if (e != cudaSuccess) return e;
         // one or two cells of the first level's larger colour per thread
-        int64_t t = (P.lv[0].cells() + 1) / 2;
+        const int64_t t = (int64_t)((P.lv[0].n[0] + 1) / 2) * P.lv[0].n[1] * P.lv[0].n[2];
         const unsigned nth = (unsigned)(t >= 512 ? 512 : (t + 31) / 32 * 32);
         ProfScope ps("k_dif_coarse", st);
         k_dif_coarse<DIM><<<1, nth, bytes, st>>>(P, bf, b0);
@@ -1056,7 +1097,7 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         size_t bytes = 0;
         while (lc > 0 && nl - lc < kDifCoarseMax) {
             bytes += dcoarse_doubles(lv[lc - 1], dim) * sizeof(double);
-            if (bytes > kDifCoarseSmem || lv[lc - 1].cells() > 32768) break;
+            if (bytes > kDifCoarseSmem || lv[lc - 1].cells() > (dim == 2 && !bc.per[0] && !bc.per[1] ? kDifCoarse2 : 32768)) break;
             lc--;
         }
     }

@@ -324,10 +324,11 @@ __global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo b
 // The coarse end of the V-cycle in one CTA: every level from the first whose arrays
 // fit shared memory (about 128^2 or 27^3 cells) down to the coarsest grid and back,
 // with a barrier between half sweeps: one launch instead of eleven per level and a
-// bottom solve.  @@MC
+// bottom solve (27 us where the bottom alone took 76).
 constexpr int kCoarseMax = 12;  // levels it may hold
 constexpr int kCoarseCells = 27000;  // cells of all of them (two floats each, 216 KB)
 constexpr int kBottomSweeps = 64;
+constexpr int64_t kCoarse2 = 1100;  // 2-D: larger levels go by legs
 struct MCoarse {
     int nl;
     CLevel lv[kCoarseMax];
@@ -339,112 +340,148 @@ template <int DIM>
 __global__ void __launch_bounds__(1024) k_mg_coarse(const __grid_constant__ MCoarse P, const __grid_constant__ BcInfo bc)
 {
     extern __shared__ float smf[];
-    __shared__ CLevel lv[kCoarseMax];
+    __shared__ int soff[kCoarseMax + 1];  // where each level's arrays begin
     const int tid = threadIdx.x, nth = blockDim.x;
+    auto level = [&](int l) {
+        CLevel L = P.lv[l];
+        const int nc = (int)L.cells();
+        L.phi = smf + soff[l];
+        L.rhs = L.phi + nc;
+        L.res = nullptr;
+        return L;
+    };
     {
-        float* p = smf;
+        int o = 0;
         for (int l = 0; l < P.nl; l++) {
             const CLevel& G = P.lv[l];
             const int nc = (int)G.cells();
-            float* phi = p;
-            float* rhs = p + nc;
-            p += 2 * nc;
+            if (tid == 0) soff[l] = o;
             for (int c = tid; c < nc; c += nth) {
-                phi[c] = 0.0f;
-                if (l == 0) rhs[c] = G.rhs[c];
+                smf[o + c] = 0.0f;
+                if (l == 0) smf[o + nc + c] = G.rhs[c];
             }
-            if (tid == 0) {
-                CLevel L = G;
-                L.phi = phi;
-                L.rhs = rhs;
-                L.res = nullptr;
-                lv[l] = L;
-            }
+            o += 2 * nc;
         }
     }
     __syncthreads();
     // c / n, exact for the sizes here (c n < 2^32)
     auto quot = [](int c, unsigned magic, int n) { return n == 1 ? c : (int)__umulhi((unsigned)c, magic); };
-    auto cell = [&](int l, int c, int& i, int& j, int& k) {
-        const int n0 = lv[l].n[0], n1 = lv[l].n[1];
+    auto cell = [&](const CLevel& L, int l, int c, int& i, int& j, int& k) {
+        const int n0 = L.n[0], n1 = L.n[1];
         const int row = DIM > 1 ? quot(c, P.m0[l], n0) : 0;
         i = DIM > 1 ? c - row * n0 : c;
         k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
         j = DIM > 2 ? row - k * n1 : row;
     };
-    // one half sweep by threads t, t + step, ... over the cells of a colour; whether
-    // a cell changed
-    auto half = [&](int l, int color, int t, int step) -> bool {
-        const CLevel& L = lv[l];
-        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2, nq = h * n1 * L.n[2];
-        bool ch = false;
-        for (int q = t; q < nq; q += step) {
-            const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
-            const int k = DIM > 2 ? quot(row, P.m1[l], n1) : 0, j = DIM > 2 ? row - k * n1 : row;
-            const int i = 2 * (q - row * h) + ((j + k + color) & 1);
-            if (i >= n0) continue;
-            const int c = i + n0 * row;
-            float off, diag;
-            stencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
-            const float v = __fdividef(L.rhs[c] - off, diag);
-            ch |= !(v == L.phi[c]);
-            L.phi[c] = v;
-        }
-        return ch;
+    // cell q of a colour: x pair fastest, then the rows; false past the row's end
+    auto colour_cell = [&](const CLevel& L, int l, int color, int q, int& i, int& j, int& k, int& c) {
+        const int n0 = L.n[0], n1 = L.n[1], h = (n0 + 1) / 2;
+        const int row = DIM > 1 ? quot(q, P.mh[l], h) : 0;
+        k = DIM > 2 ? quot(row, P.m1[l], n1) : 0;
+        j = DIM > 2 ? row - k * n1 : row;
+        i = 2 * (q - row * h) + ((j + k + color) & 1);
+        c = i + n0 * row;
+        return i < n0;
     };
-    for (int l = 0; l < P.nl - 1; l++) {
+    auto sweeps2 = [&](const CLevel& L, int l) {
+        const int nq = (L.n[0] + 1) / 2 * L.n[1] * L.n[2];
         for (int s = 0; s < 4; s++) {
-            half(l, s & 1, tid, nth);
+            for (int q = tid; q < nq; q += nth) {
+                int i, j, k, c;
+                if (!colour_cell(L, l, s & 1, q, i, j, k, c)) continue;
+                float off, diag;
+                stencil<DIM>(L, bc, i, j, k, L.phi, off, diag);
+                L.phi[c] = __fdividef(L.rhs[c] - off, diag);
+            }
             __syncthreads();
         }
-        const CLevel& C = lv[l + 1];
+    };
+    for (int l = 0; l < P.nl - 1; l++) {
+        const CLevel F = level(l), C = level(l + 1);
+        sweeps2(F, l);
         const int nc = (int)C.cells();
         for (int c = tid; c < nc; c += nth) {
             int i, j, k;
-            cell(l + 1, c, i, j, k);
-            C.rhs[c] = mg_restrict<DIM>(lv[l], bc, i, j, k);
+            cell(C, l + 1, c, i, j, k);
+            C.rhs[c] = mg_restrict<DIM>(F, bc, i, j, k);
         }
         __syncthreads();
     }
     {
-        // ends early once a whole sweep changes nothing (every later one would repeat it)
+        // Bottom solve.  Up to one cell of each colour per thread: its neighbours' places,
+        // their coefficients (0 beyond a domain face, whose value is 0 on a correction
+        // level), the diagonal and the right-hand side stay in registers, and only the
+        // warps that hold cells take part (one warp: no barrier, and it ends once a
+        // whole sweep changes nothing, as every later one would repeat it).
         const int l = P.nl - 1;
-        if ((int)lv[l].cells() <= 64) {
-            if (tid < 32) {
+        const CLevel L = level(l);
+        const int nq = (L.n[0] + 1) / 2 * L.n[1] * L.n[2];
+        if (nq <= nth) {
+            const int nb = (nq + 31) / 32 * 32;
+            if (tid < nb) {
+                float* at[2];
+                int lo[2][DIM], hi[2][DIM];
+                float wl[2][DIM], wh[2][DIM], diag[2], r[2];
+                bool ok[2];
+#pragma unroll
+                for (int color = 0; color < 2; color++) {
+                    int i, j, k, c;
+                    ok[color] = colour_cell(L, l, color, tid, i, j, k, c) && tid < nq;
+                    if (!ok[color]) continue;
+                    at[color] = L.phi + c;
+                    r[color] = L.rhs[c];
+                    float off;
+                    stencil<DIM>(L, bc, i, j, k, L.phi, off, diag[color]);
+                    const int cc[3] = {i, j, k}, str[3] = {1, L.n[0], L.n[0] * L.n[1]};
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) {
+                        const bool l1 = cc[d] > 0, h1 = cc[d] < L.n[d] - 1;
+                        lo[color][d] = l1 ? -str[d] : 0;
+                        hi[color][d] = h1 ? str[d] : 0;
+                        wl[color][d] = l1 ? (float)L.idx2[d] : 0.0f;
+                        wh[color][d] = h1 ? (float)L.idx2[d] : 0.0f;
+                    }
+                }
                 for (int s = 0; s < kBottomSweeps; s++) {
-                    bool ch = half(l, 0, tid, 32);
-                    __syncwarp();
-                    ch |= half(l, 1, tid, 32);
-                    __syncwarp();
-                    if (!__any_sync(0xffffffffu, ch)) break;
+                    bool ch = false;
+#pragma unroll
+                    for (int color = 0; color < 2; color++) {
+                        if (ok[color]) {
+                            float off = 0;
+#pragma unroll
+                            for (int d = 0; d < DIM; d++) {
+                                off = fmaf(wl[color][d], at[color][lo[color][d]], off);
+                                off = fmaf(wh[color][d], at[color][hi[color][d]], off);
+                            }
+                            const float v = __fdividef(r[color] - off, diag[color]);
+                            ch |= !(v == *at[color]);
+                            *at[color] = v;
+                        }
+                        if (nb == 32) __syncwarp();
+                        else asm volatile("bar.sync 1, %0;" ::"r"(nb) : "memory");
+                    }
+                    if (nb == 32 && !__any_sync(0xffffffffu, ch)) break;
                 }
             }
             __syncthreads();
         } else {
-            for (int s = 0; s < kBottomSweeps; s++) {
-                bool ch = half(l, 0, tid, nth);
-                __syncthreads();
-                ch |= half(l, 1, tid, nth);
-                if (!__syncthreads_or(ch)) break;
-            }
+            for (int s = 0; s < kBottomSweeps / 2; s++) sweeps2(L, l);
         }
     }
     for (int l = P.nl - 2; l >= 0; l--) {
-        const CLevel& F = lv[l];
+        const CLevel F = level(l), C = level(l + 1);
         const int nc = (int)F.cells();
         for (int c = tid; c < nc; c += nth) {
             int i, j, k;
-            cell(l, c, i, j, k);
-            F.phi[c] += mg_prolong<DIM>(lv[l + 1], bc, i, j, k);
+            cell(F, l, c, i, j, k);
+            F.phi[c] += mg_prolong<DIM>(C, bc, i, j, k);
         }
         __syncthreads();
-        for (int s = 0; s < 4; s++) {
-            half(l, s & 1, tid, nth);
-            __syncthreads();
-        }
+        sweeps2(F, l);
     }
-    const int nc = (int)lv[0].cells();
-    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = lv[0].phi[c];
+    const CLevel L0 = level(0);
+    const int nc = (int)L0.cells();
+    for (int c = tid; c < nc; c += nth) P.lv[0].phi[c] = L0.phi[c];
 }
 
 // the operator of a 2-D correction level as the fused legs take it (vd_mg2d.cuh)
@@ -508,7 +545,7 @@ struct Mg {
         cudaError_t e = cudaFuncSetAttribute(k_mg_coarse<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              kCoarseCells * 2 * (int)sizeof(float));
         if (e != cudaSuccess) return e;
-        int64_t t = (P.lv[0].cells() + 1) / 2;
+        const int64_t t = (int64_t)((P.lv[0].n[0] + 1) / 2) * P.lv[0].n[1] * P.lv[0].n[2];
         const unsigned nth = (unsigned)(t >= 1024 ? 1024 : (t + 31) / 32 * 32);
         ProfScope ps("k_mg_coarse", st);
         k_mg_coarse<DIM><<<1, nth, 2 * cells * sizeof(float), st>>>(P, b);
@@ -842,7 +879,7 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         int64_t cells = 0;
         while (lc > 0 && nl - lc < kCoarseMax) {
             cells += lv[lc - 1].cells();
-            if (cells > kCoarseCells) break;
+            if (cells > kCoarseCells || (dim == 2 && lv[lc - 1].cells() > kCoarse2)) break;
             lc--;
         }
     }
