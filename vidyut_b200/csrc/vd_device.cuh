@@ -239,65 +239,125 @@ __device__ __forceinline__ R gk_map(R wk, R g)
 // 13/12 and 1/4) and eps4 is 4 eps: every weight is a ratio of these, and scaling
 // by a power of two changes no rounding, so the result is the same and each
 // indicator costs one multiply less.
-__device__ __forceinline__ float weno_weights_f32(float b1, float b2, float b3, float p1, float p2, float p3, int scheme,
-                                                  float eps4)
+// Two FP32 values in one register pair: Blackwell's packed FP32 arithmetic (one issue
+// slot for both halves, each rounded as the scalar operation).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 pack2(float x, float y)
 {
-    const float q1 = b1 + eps4, q2 = b2 + eps4, q3 = b3 + eps4;
-    const float m = fminf(q1, fminf(q2, q3));
-    const float r1 = rcp_approx(q1), r2 = rcp_approx(q2), r3 = rcp_approx(q3);
-    float a1, a2, a3;
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void unpack2(F2 a, float& x, float& y)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+}
+__device__ __forceinline__ F2 both2(float x) { return pack2(x, x); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) { return fma2(both2(-1.0f), b, a); }  // one rounding, as a - b
+
+// One reconstruction of two fields at once (packed), eps4 the same for both; scheme 3
+// WENO-Z, 1 WENO-JS, 2 WENO-M.  The kernel is issue bound (72 % active, FMA 35 %): the
+// drift flux and the density of a face go through packed operations side by side, same
+// bits (B200: 3-D transport of 24 species on 128^3 1.86 -> 1.80 ms, a batched 2-D
+// step 0.295 -> 0.276 ms).
+__device__ __forceinline__ F2 weno_weights_f32(F2 b1, F2 b2, F2 b3, F2 p1, F2 p2, F2 p3, int scheme, F2 eps4)
+{
+    const F2 q1 = add2(b1, eps4), q2 = add2(b2, eps4), q3 = add2(b3, eps4);
+    float q1x, q1y, q2x, q2y, q3x, q3y;
+    unpack2(q1, q1x, q1y);
+    unpack2(q2, q2x, q2y);
+    unpack2(q3, q3x, q3y);
+    const float mx = fminf(q1x, fminf(q2x, q3x)), my = fminf(q1y, fminf(q2y, q3y));
+    const F2 r1 = pack2(rcp_approx(q1x), rcp_approx(q1y)), r2 = pack2(rcp_approx(q2x), rcp_approx(q2y));
+    const F2 r3 = pack2(rcp_approx(q3x), rcp_approx(q3y));
+    F2 a1, a2, a3;
     if (scheme == 3) {
-        const float tau = fabsf(b1 - b3);
-        const bool big = tau > m;
-        const float cr = big ? m * rcp_approx(tau) : 1.0f;
-        const float t = big ? m : tau;
-        const float B1 = t * r1, B2 = t * r2, B3 = t * r3;
-        const float c2 = cr * cr;
-        a1 = 0.1f * fmaf(B1, B1, c2);
-        a2 = 0.6f * fmaf(B2, B2, c2);
-        a3 = 0.3f * fmaf(B3, B3, c2);
+        float tx, ty;
+        unpack2(sub2(b1, b3), tx, ty);
+        tx = fabsf(tx);
+        ty = fabsf(ty);
+        const bool bx = tx > mx, by = ty > my;
+        const float cx = bx ? __fmul_rn(mx, rcp_approx(tx)) : 1.0f, cy = by ? __fmul_rn(my, rcp_approx(ty)) : 1.0f;
+        const F2 t = pack2(bx ? mx : tx, by ? my : ty), cr = pack2(cx, cy);
+        const F2 B1 = mul2(t, r1), B2 = mul2(t, r2), B3 = mul2(t, r3);
+        const F2 c2 = mul2(cr, cr);
+        a1 = mul2(both2(0.1f), fma2(B1, B1, c2));
+        a2 = mul2(both2(0.6f), fma2(B2, B2, c2));
+        a3 = mul2(both2(0.3f), fma2(B3, B3, c2));
     } else {
-        const float B1 = m * r1, B2 = m * r2, B3 = m * r3;
-        a1 = 0.1f * (B1 * B1);
-        a2 = 0.6f * (B2 * B2);
-        a3 = 0.3f * (B3 * B3);
+        const F2 m = pack2(mx, my);
+        const F2 B1 = mul2(m, r1), B2 = mul2(m, r2), B3 = mul2(m, r3);
+        a1 = mul2(both2(0.1f), mul2(B1, B1));
+        a2 = mul2(both2(0.6f), mul2(B2, B2));
+        a3 = mul2(both2(0.3f), mul2(B3, B3));
         if (scheme == 2) {
-            const float is = rcp_approx(a1 + a2 + a3);
-            a1 = gk_map(a1 * is, 0.1f);
-            a2 = gk_map(a2 * is, 0.6f);
-            a3 = gk_map(a3 * is, 0.3f);
+            float x, y, ax, ay;
+            unpack2(add2(add2(a1, a2), a3), x, y);
+            x = rcp_approx(x);
+            y = rcp_approx(y);
+            unpack2(a1, ax, ay);
+            a1 = pack2(gk_map(ax * x, 0.1f), gk_map(ay * y, 0.1f));
+            unpack2(a2, ax, ay);
+            a2 = pack2(gk_map(ax * x, 0.6f), gk_map(ay * y, 0.6f));
+            unpack2(a3, ax, ay);
+            a3 = pack2(gk_map(ax * x, 0.3f), gk_map(ay * y, 0.3f));
         }
     }
-    return fmaf(a1, p1, fmaf(a2, p2, a3 * p3)) * rcp_approx(a1 + a2 + a3);
+    float sx, sy;
+    unpack2(add2(add2(a1, a2), a3), sx, sy);
+    return mul2(fma2(a1, p1, fma2(a2, p2, mul2(a3, p3))), pack2(rcp_approx(sx), rcp_approx(sy)));
 }
 
-// Both reconstructions of one field at a face from its six stencil values x0..x5:
+// Both reconstructions of two fields at a face from their six stencil values x0..x5:
 // plus, the left-biased WENO-5 value from x0..x4, and minus, the right-biased one
 // from x5..x1 (weno(e,d,c,b,a) of the reference).
 // They share two of their three second differences (x1-2x2+x3, x2-2x3+x4) with
 // their squared terms, and two of their candidate polynomials (the parabola
 // through x1..x3 at x2+1/2 and through x2..x4 at x3+1/2), which are computed once.
-__device__ __forceinline__ void weno_pair_f32(const float* x, int scheme, float eps4, float& plus, float& minus)
+__device__ __forceinline__ void weno_pair_f32(const F2* x, int scheme, F2 eps4, F2& plus, F2& minus)
 {
+    const F2 k2 = both2(-2.0f), k133 = both2(13.0f / 3.0f), k13 = both2(1.0f / 3.0f), k56 = both2(5.0f / 6.0f);
+    const F2 k16 = both2(-1.0f / 6.0f), k76 = both2(-7.0f / 6.0f), k116 = both2(11.0f / 6.0f);
+    const F2 k3 = both2(3.0f), k4 = both2(-4.0f);
     // second differences and the 13/3 d^2 terms of the windows centred at x1..x4
-    const float d1 = fmaf(-2.0f, x[1], x[0]) + x[2], d2 = fmaf(-2.0f, x[2], x[1]) + x[3];
-    const float d3 = fmaf(-2.0f, x[3], x[2]) + x[4], d4 = fmaf(-2.0f, x[4], x[3]) + x[5];
-    const float c2 = (13.0f / 3.0f) * (d2 * d2), c3 = (13.0f / 3.0f) * (d3 * d3);
+    const F2 d1 = add2(fma2(k2, x[1], x[0]), x[2]), d2 = add2(fma2(k2, x[2], x[1]), x[3]);
+    const F2 d3 = add2(fma2(k2, x[3], x[2]), x[4]), d4 = add2(fma2(k2, x[4], x[3]), x[5]);
+    const F2 c2 = mul2(k133, mul2(d2, d2)), c3 = mul2(k133, mul2(d3, d3));
     // the polynomials the two share
-    const float pm = fmaf(-1.0f / 6.0f, x[1], fmaf(5.0f / 6.0f, x[2], (1.0f / 3.0f) * x[3]));
-    const float pn = fmaf(1.0f / 3.0f, x[2], fmaf(5.0f / 6.0f, x[3], (-1.0f / 6.0f) * x[4]));
+    const F2 pm = fma2(k16, x[1], fma2(k56, x[2], mul2(k13, x[3])));
+    const F2 pn = fma2(k13, x[2], fma2(k56, x[3], mul2(k16, x[4])));
     {
-        const float p1 = fmaf(1.0f / 3.0f, x[0], fmaf(-7.0f / 6.0f, x[1], (11.0f / 6.0f) * x[2]));
-        const float t2 = fmaf(3.0f, x[2], fmaf(-4.0f, x[1], x[0])), t4 = x[1] - x[3];
-        const float t6 = fmaf(3.0f, x[2], fmaf(-4.0f, x[3], x[4]));
-        const float b1 = fmaf(13.0f / 3.0f, d1 * d1, t2 * t2), b2 = fmaf(t4, t4, c2), b3 = fmaf(t6, t6, c3);
+        const F2 p1 = fma2(k13, x[0], fma2(k76, x[1], mul2(k116, x[2])));
+        const F2 t2 = fma2(k3, x[2], fma2(k4, x[1], x[0])), t4 = sub2(x[1], x[3]);
+        const F2 t6 = fma2(k3, x[2], fma2(k4, x[3], x[4]));
+        const F2 b1 = fma2(k133, mul2(d1, d1), mul2(t2, t2)), b2 = fma2(t4, t4, c2), b3 = fma2(t6, t6, c3);
         plus = weno_weights_f32(b1, b2, b3, p1, pm, pn, scheme, eps4);
     }
     {
-        const float p1 = fmaf(1.0f / 3.0f, x[5], fmaf(-7.0f / 6.0f, x[4], (11.0f / 6.0f) * x[3]));
-        const float t2 = fmaf(3.0f, x[3], fmaf(-4.0f, x[4], x[5])), t4 = x[4] - x[2];
-        const float t6 = fmaf(3.0f, x[3], fmaf(-4.0f, x[2], x[1]));
-        const float b1 = fmaf(13.0f / 3.0f, d4 * d4, t2 * t2), b2 = fmaf(t4, t4, c3), b3 = fmaf(t6, t6, c2);
+        const F2 p1 = fma2(k13, x[5], fma2(k76, x[4], mul2(k116, x[3])));
+        const F2 t2 = fma2(k3, x[3], fma2(k4, x[4], x[5])), t4 = sub2(x[4], x[2]);
+        const F2 t6 = fma2(k3, x[3], fma2(k4, x[2], x[1]));
+        const F2 b1 = fma2(k133, mul2(d4, d4), mul2(t2, t2)), b2 = fma2(t4, t4, c3), b3 = fma2(t6, t6, c2);
         minus = weno_weights_f32(b1, b2, b3, p1, pn, pm, scheme, eps4);
     }
 }
@@ -342,16 +402,19 @@ __device__ __forceinline__ float face_flux_mixed32(const float* u, const float* 
     b2 = b2 < 0 ? 0 : (b2 > 255 ? 255 : b2);
     const float s2 = __int_as_float(b2 << 23);        // 2^-2e, 0 or inf at the ends
     const float eps = 4.0f * fminf(fmaxf(1e-20f * s2, 1e-30f), 1e30f);  // the weights take 4 eps
-    float us[6], fs[6];
+    // the drift flux f = u v in the low half, the density in the high half
+    F2 x[6];
 #pragma unroll
     for (int q = 0; q < 6; q++) {
-        us[q] = u[q] * s;
-        fs[q] = us[q] * v[q];
+        const float us = __fmul_rn(u[q], s);
+        x[q] = pack2(__fmul_rn(us, v[q]), us);
     }
-    const float lam = fabsf(0.5f * (v[2] + v[3]));
+    const float lam = fabsf(__fmul_rn(0.5f, __fadd_rn(v[2], v[3])));
+    F2 plus, minus;
+    weno_pair_f32(x, scheme, both2(eps), plus, minus);
     float fp, fm, up, um;
-    weno_pair_f32(fs, scheme, eps, fp, fm);
-    weno_pair_f32(us, scheme, eps, up, um);
+    unpack2(plus, fp, up);
+    unpack2(minus, fm, um);
     const float F = 0.5f * (fmaf(lam, up, fp) + fmaf(-lam, um, fm));
     if (bs < 254) return F * __int_as_float((254 - bs) << 23);  // 2^(127-bs)
     return (float)((double)F * __longlong_as_double((long long)(1150 - bs) << 52));

@@ -860,7 +860,13 @@ int tune_get(const char* key)
 template <int DIM, int PREC>
 static cudaError_t launch_tr_v(const TransportArgs& a, cudaStream_t st)
 {
-    const int mb = g_tr_minb[DIM][PREC];
+    int mb = g_tr_minb[DIM][PREC];
+    // Where two CTAs per SM hold every tile there is nothing for more to overlap, and
+    // the variants for fewer have the registers (200 x 150: FP64 21.0 us for 25.4 us,
+    // mixed 27.1 for 29.9); with more tiles the tuned one wins (467 x 509, 960
+    // tiles: FP64 74 for 79 us, mixed 83 for 94).
+    const int64_t ntiles = (int64_t)a.ntile[0] * a.ntile[1] * a.ntile[2];
+    if (DIM < 3 && ntiles <= 2 * 148 && mb > 2) mb = 2;
     if constexpr (DIM < 3) {
         if (mb == 4) return launch_tr<DIM, PREC, 4>(a, st);
         if (mb == 3) return launch_tr<DIM, PREC, 3>(a, st);
@@ -917,6 +923,7 @@ static cudaError_t load_update_kernels()
         if (mb == 4) fn = (const void*)k_transport<DIM, PREC, 4>;
     }
     cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e == cudaSuccess && mb > 2) e = cudaFuncGetAttributes(&fa, (const void*)k_transport<DIM, PREC, 2>);  // small boxes
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, (const void*)k_joule_pre<DIM, PREC>);
     return e;
 }
