@@ -182,6 +182,7 @@ __device__ __forceinline__ void dstencil(const DLevel& L, const DBc& bc, int i, 
 template <int DIM>
 __global__ void __launch_bounds__(128) k_dif_rbgs(DLevel L, DBc bc, int color, int half)
 {
+    grid_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     int ii[2], jj[2], kk[2];
     bool ok[2];
@@ -215,6 +216,7 @@ __global__ void __launch_bounds__(128) k_dif_rbgs(DLevel L, DBc bc, int color, i
 template <int DIM>
 __global__ void __launch_bounds__(128) k_dif_residual(DLevel L, DBc bc, double* blkmax)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double m = 0.0;
@@ -261,6 +263,7 @@ __device__ __forceinline__ double drestrict(const DLevel& F, const DBc& bc, int 
 template <int DIM>
 __global__ void __launch_bounds__(128) k_dif_restrict(DLevel F, DLevel C, DBc bc)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C.n[0]) return;
@@ -274,6 +277,7 @@ __global__ void __launch_bounds__(128) k_dif_restrict(DLevel F, DLevel C, DBc bc
 template <int DIM, int D>
 __global__ void __launch_bounds__(128) k_dif_coarsen_b(DLevel F, DLevel C)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C.n[0] + (D == 0)) return;
@@ -361,6 +365,7 @@ __device__ __forceinline__ double dprolong(const DLevel& C, const DBc& bc, int i
 template <int DIM>
 __global__ void __launch_bounds__(128) k_dif_prolong(DLevel F, DLevel C, DBc bc)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n[0]) return;
@@ -395,6 +400,7 @@ template <int DIM>
 __global__ void __launch_bounds__(512) k_dif_coarse(const __grid_constant__ DCoarse P, const __grid_constant__ DBc bcf,
                                                      const __grid_constant__ DBc bc0)
 {
+    grid_wait();
     extern __shared__ double sm[];
     __shared__ int soff[kDifCoarseMax + 1];  // where each level's arrays begin
     const int tid = threadIdx.x, nth = blockDim.x;
@@ -577,6 +583,7 @@ struct DOp2 {
 
 __global__ void k_dif_maxabs(const double* x, int64_t n, unsigned long long* out)
 {
+    grid_wait();
     double m = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
         m = fmax(m, fabs(x[c]));
@@ -601,6 +608,7 @@ struct DifArgs {
 template <int DIM>
 __global__ void __launch_bounds__(128) k_dif_cell_d(DifArgs a, double* Dg, int g0, int g1)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g0) return;
@@ -623,6 +631,7 @@ __global__ void __launch_bounds__(128) k_dif_cell_d(DifArgs a, double* Dg, int g
 template <int DIM, int D>
 __global__ void __launch_bounds__(128) k_dif_face_b(DLevel L, const double* Dg, int g0, int g1)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= L.n[0] + (D == 0)) return;
@@ -639,6 +648,7 @@ __global__ void __launch_bounds__(128) k_dif_face_b(DLevel L, const double* Dg, 
 template <int DIM, int D>
 __global__ void __launch_bounds__(128) k_dif_bcval(DifArgs a, DLevel L, double* out, int sgn)
 {
+    grid_wait();
     constexpr int E0 = D == 0 ? 1 : 0, E1 = D == 2 ? 1 : 2;
     const int t0 = blockIdx.x * blockDim.x + threadIdx.x, t1 = blockIdx.y;
     if (t0 >= L.n[E0] || t1 >= L.n[E1]) return;
@@ -685,6 +695,7 @@ __global__ void __launch_bounds__(128) k_dif_bcval(DifArgs a, DLevel L, double* 
 // rhs = n_old/dt + dsdt; initial guess = the current state
 __global__ void __launch_bounds__(128) k_dif_rhs(DifArgs a, DLevel L)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= L.n[0]) return;
@@ -697,6 +708,7 @@ __global__ void __launch_bounds__(128) k_dif_rhs(DifArgs a, DLevel L)
 // floor, copy to the output; the electron energy's Te update and floor
 __global__ void __launch_bounds__(128) k_dif_finish(DifArgs a, DLevel L)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= L.n[0]) return;
@@ -725,6 +737,7 @@ __global__ void __launch_bounds__(128) k_dif_finish(DifArgs a, DLevel L)
 template <int D>
 __global__ void __launch_bounds__(128) k_dif_grad(DLevel L, DBc bc, A4 out, int lo0, int lo1, int lo2)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= L.n[0] + (D == 0)) return;
@@ -789,22 +802,22 @@ struct DifOps {
         dim3 g = dgrid(L, 0, 2);
         if (DIM == 3) g.z = (unsigned)half;
         else if (DIM == 2) g.y = (unsigned)half;
-        k_dif_rbgs<DIM><<<g, 128, 0, st>>>(L, b, color, half);
+        launch_after(k_dif_rbgs<DIM>, g, 128, 0, st, L, b, color, half);
     }
     static void residual(const DLevel& L, const DBc& b, double* mx, cudaStream_t st)
     {
         ProfScope ps("k_dif_residual", st);
-        k_dif_residual<DIM><<<dgrid(L), 128, 0, st>>>(L, b, mx);
+        launch_after(k_dif_residual<DIM>, dgrid(L), 128, 0, st, L, b, mx);
     }
     static void restrict_(const DLevel& F, const DLevel& C, const DBc& b, cudaStream_t st)
     {
         ProfScope ps("k_dif_restrict", st);
-        k_dif_restrict<DIM><<<dgrid(C), 128, 0, st>>>(F, C, b);
+        launch_after(k_dif_restrict<DIM>, dgrid(C), 128, 0, st, F, C, b);
     }
     static void prolong(const DLevel& F, const DLevel& C, const DBc& b, cudaStream_t st)
     {
         ProfScope ps("k_dif_prolong", st);
-        k_dif_prolong<DIM><<<dgrid(F), 128, 0, st>>>(F, C, b);
+        launch_after(k_dif_prolong<DIM>, dgrid(F), 128, 0, st, F, C, b);
     }
     static cudaError_t coarse(const DCoarse& P, const DBc& bf, const DBc& b0, cudaStream_t st)
     {
@@ -817,44 +830,44 @@ struct DifOps {
         const int64_t t = (int64_t)((P.lv[0].n[0] + 1) / 2) * P.lv[0].n[1] * P.lv[0].n[2];
         const unsigned nth = (unsigned)(t >= 512 ? 512 : (t + 31) / 32 * 32);
         ProfScope ps("k_dif_coarse", st);
-        k_dif_coarse<DIM><<<1, nth, bytes, st>>>(P, bf, b0);
+        launch_after(k_dif_coarse<DIM>, 1, nth, bytes, st, P, bf, b0);
         return cudaGetLastError();
     }
     static void coarsen_b(const DLevel& F, const DLevel& C, cudaStream_t st)
     {
         ProfScope ps("k_dif_coarsen_b", st);
-        k_dif_coarsen_b<DIM, 0><<<dgrid(C, 1), 128, 0, st>>>(F, C);
-        if (DIM > 1) k_dif_coarsen_b<DIM, (DIM > 1 ? 1 : 0)><<<dim3((C.n[0] + 127) / 128, C.n[1] + 1, C.n[2]), 128, 0, st>>>(F, C);
-        if (DIM > 2) k_dif_coarsen_b<DIM, (DIM > 2 ? 2 : 0)><<<dim3((C.n[0] + 127) / 128, C.n[1], C.n[2] + 1), 128, 0, st>>>(F, C);
+        launch_after(k_dif_coarsen_b<DIM, 0>, dgrid(C, 1), 128, 0, st, F, C);
+        if (DIM > 1) launch_after(k_dif_coarsen_b<DIM, (DIM > 1 ? 1 : 0)>, dim3((C.n[0] + 127) / 128, C.n[1] + 1, C.n[2]), 128, 0, st, F, C);
+        if (DIM > 2) launch_after(k_dif_coarsen_b<DIM, (DIM > 2 ? 2 : 0)>, dim3((C.n[0] + 127) / 128, C.n[1], C.n[2] + 1), 128, 0, st, F, C);
     }
     static void setup(const DifArgs& a, const DLevel& L0, double* Dg, double* const bv_lo[3], double* const bv_hi[3],
                       cudaStream_t st)
     {
         const int g0 = L0.n[0] + 2, g1 = L0.n[1] + (DIM > 1 ? 2 : 0), g2 = L0.n[2] + (DIM > 2 ? 2 : 0);
         ProfScope ps("k_dif_setup", st);
-        k_dif_cell_d<DIM><<<dim3((g0 + 127) / 128, g1, g2), 128, 0, st>>>(a, Dg, g0, g1);
-        k_dif_face_b<DIM, 0><<<dgrid(L0, 1), 128, 0, st>>>(L0, Dg, g0, g1);
+        launch_after(k_dif_cell_d<DIM>, dim3((g0 + 127) / 128, g1, g2), 128, 0, st, a, Dg, g0, g1);
+        launch_after(k_dif_face_b<DIM, 0>, dgrid(L0, 1), 128, 0, st, L0, Dg, g0, g1);
         if (DIM > 1)
-            k_dif_face_b<DIM, (DIM > 1 ? 1 : 0)><<<dim3((L0.n[0] + 127) / 128, L0.n[1] + 1, L0.n[2]), 128, 0, st>>>(
+            launch_after(k_dif_face_b<DIM, (DIM > 1 ? 1 : 0)>, dim3((L0.n[0] + 127) / 128, L0.n[1] + 1, L0.n[2]), 128, 0, st, 
                 L0, Dg, g0, g1);
         if (DIM > 2)
-            k_dif_face_b<DIM, (DIM > 2 ? 2 : 0)><<<dim3((L0.n[0] + 127) / 128, L0.n[1], L0.n[2] + 1), 128, 0, st>>>(
+            launch_after(k_dif_face_b<DIM, (DIM > 2 ? 2 : 0)>, dim3((L0.n[0] + 127) / 128, L0.n[1], L0.n[2] + 1), 128, 0, st, 
                 L0, Dg, g0, g1);
         for (int d = 0; d < DIM; d++) {
             const int e0 = d == 0 ? 1 : 0, e1 = d == 2 ? 1 : 2;
             const dim3 g((unsigned)((L0.n[e0] + 127) / 128), (unsigned)L0.n[e1]);
             if (d == 0) {
-                if (bv_lo[0]) k_dif_bcval<DIM, 0><<<g, 128, 0, st>>>(a, L0, bv_lo[0], -1);
-                if (bv_hi[0]) k_dif_bcval<DIM, 0><<<g, 128, 0, st>>>(a, L0, bv_hi[0], 1);
+                if (bv_lo[0]) launch_after(k_dif_bcval<DIM, 0>, g, 128, 0, st, a, L0, bv_lo[0], -1);
+                if (bv_hi[0]) launch_after(k_dif_bcval<DIM, 0>, g, 128, 0, st, a, L0, bv_hi[0], 1);
             } else if (d == 1) {
-                if (bv_lo[1]) k_dif_bcval<DIM, (DIM > 1 ? 1 : 0)><<<g, 128, 0, st>>>(a, L0, bv_lo[1], -1);
-                if (bv_hi[1]) k_dif_bcval<DIM, (DIM > 1 ? 1 : 0)><<<g, 128, 0, st>>>(a, L0, bv_hi[1], 1);
+                if (bv_lo[1]) launch_after(k_dif_bcval<DIM, (DIM > 1 ? 1 : 0)>, g, 128, 0, st, a, L0, bv_lo[1], -1);
+                if (bv_hi[1]) launch_after(k_dif_bcval<DIM, (DIM > 1 ? 1 : 0)>, g, 128, 0, st, a, L0, bv_hi[1], 1);
             } else {
-                if (bv_lo[2]) k_dif_bcval<DIM, (DIM > 2 ? 2 : 0)><<<g, 128, 0, st>>>(a, L0, bv_lo[2], -1);
-                if (bv_hi[2]) k_dif_bcval<DIM, (DIM > 2 ? 2 : 0)><<<g, 128, 0, st>>>(a, L0, bv_hi[2], 1);
+                if (bv_lo[2]) launch_after(k_dif_bcval<DIM, (DIM > 2 ? 2 : 0)>, g, 128, 0, st, a, L0, bv_lo[2], -1);
+                if (bv_hi[2]) launch_after(k_dif_bcval<DIM, (DIM > 2 ? 2 : 0)>, g, 128, 0, st, a, L0, bv_hi[2], 1);
             }
         }
-        k_dif_rhs<<<dgrid(L0), 128, 0, st>>>(a, L0);
+        launch_after(k_dif_rhs, dgrid(L0), 128, 0, st, a, L0);
     }
 };
 
@@ -1126,8 +1139,8 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
         op.bcc = bc0;
         ProfScope ps(up ? "k_dif_leg_up" : "k_dif_leg_down", st);
         const dim3 g = mg2d_grid(op.n);
-        if (up) k_mg2d<DOp2, true><<<g, kMg2Threads, 0, st>>>(op, lv[l].res, lv[l].phi, nullptr, mx);
-        else k_mg2d<DOp2, false><<<g, kMg2Threads, 0, st>>>(op, l == 0 ? lv[l].phi : nullptr, lv[l].res, nullptr, nullptr);
+        if (up) launch_after(k_mg2d<DOp2, true>, g, kMg2Threads, 0, st, op, lv[l].res, lv[l].phi, nullptr, mx);
+        else launch_after(k_mg2d<DOp2, false>, g, kMg2Threads, 0, st, op, l == 0 ? lv[l].phi : nullptr, lv[l].res, nullptr, nullptr);
     };
     const bool leg0 = legs && lc > 0 && nl > 1;  // the finest level goes by legs
     // mx (leg0 only): the residual's maximum, formed by the last leg
@@ -1167,12 +1180,12 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
             ops.residual(lv[0], bc, blkmax, st);
             ProfScope ps("k_dif_maxabs", st);
             const unsigned g = (unsigned)std::min<int64_t>((nblk0 + 255) / 256, 148 * 32);
-            k_dif_maxabs<<<g < 1 ? 1 : g, 256, 0, st>>>(blkmax, nblk0, d_max);
+            launch_after(k_dif_maxabs, g < 1 ? 1 : g, 256, 0, st, blkmax, nblk0, d_max);
         } else {
             ProfScope ps("k_dif_maxabs", st);
             const int64_t nc = lv[0].cells();
             unsigned g = (unsigned)std::min<int64_t>((nc + 255) / 256, 148 * 32);
-            k_dif_maxabs<<<g < 1 ? 1 : g, 256, 0, st>>>(lv[0].rhs, nc, d_max);
+            launch_after(k_dif_maxabs, g < 1 ? 1 : g, 256, 0, st, lv[0].rhs, nc, d_max);
         }
         unsigned long long h = 0;
         cudaError_t ce = cudaMemcpyAsync(&h, d_max, sizeof(h), cudaMemcpyDeviceToHost, st);
@@ -1210,15 +1223,15 @@ extern "C" int vd_implicit_species_solve(const vd_box* bx, vd_array4 state, vd_a
     }
     {
         ProfScope ps("k_dif_finish", st);
-        k_dif_finish<<<dgrid(lv[0]), 128, 0, st>>>(a, lv[0]);
+        launch_after(k_dif_finish, dgrid(lv[0]), 128, 0, st, a, lv[0]);
         if (want_grad) {
             const DLevel& L0 = lv[0];
-            k_dif_grad<0><<<dgrid(L0, 1), 128, 0, st>>>(L0, bc, A4(gradne_fc[0]), bx->lo[0], bx->lo[1], bx->lo[2]);
+            launch_after(k_dif_grad<0>, dgrid(L0, 1), 128, 0, st, L0, bc, A4(gradne_fc[0]), bx->lo[0], bx->lo[1], bx->lo[2]);
             if (dim > 1)
-                k_dif_grad<1><<<dim3((L0.n[0] + 127) / 128, L0.n[1] + 1, L0.n[2]), 128, 0, st>>>(
+                launch_after(k_dif_grad<1>, dim3((L0.n[0] + 127) / 128, L0.n[1] + 1, L0.n[2]), 128, 0, st, 
                     L0, bc, A4(gradne_fc[1]), bx->lo[0], bx->lo[1], bx->lo[2]);
             if (dim > 2)
-                k_dif_grad<2><<<dim3((L0.n[0] + 127) / 128, L0.n[1], L0.n[2] + 1), 128, 0, st>>>(
+                launch_after(k_dif_grad<2>, dim3((L0.n[0] + 127) / 128, L0.n[1], L0.n[2] + 1), 128, 0, st, 
                     L0, bc, A4(gradne_fc[2]), bx->lo[0], bx->lo[1], bx->lo[2]);
         }
     }

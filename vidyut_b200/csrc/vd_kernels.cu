@@ -235,6 +235,7 @@ struct FaceFluxArgs {
 template <int DIR, int L, int W>
 __global__ void __launch_bounds__(256) k_face_flux(const __grid_constant__ FaceFluxArgs a)
 {
+    grid_wait();
     constexpr int NC = L + 5;  // cells f0 - 3 .. f0 + L + 1 of a line
     __shared__ double su[NC * W], sv[NC * W];
     const int H = a.hyp_order == 5 ? 3 : a.hyp_order;
@@ -355,13 +356,13 @@ cudaError_t launch_face_flux(const BoxIdx& fb, int dir, int specid, const A4& ph
     // (1.3 staged cells per face instead of 1.6)
     const bool tall = (int64_t)up(fb.n[0], 32) * up(fb.n[dir], 16) * fb.n[dir == 1 ? 2 : 1] >= 2 * 148;
     if (dir == 0) {
-        k_face_flux<0, 32, 8><<<dim3(up((int64_t)fb.n[1] * fb.n[2], 8), up(fb.n[0], 32)), 256, 0, st>>>(a);
+        launch_after(k_face_flux<0, 32, 8>, dim3(up((int64_t)fb.n[1] * fb.n[2], 8), up(fb.n[0], 32)), 256, 0, st, a);
     } else if (dir == 1) {
-        if (tall) k_face_flux<1, 16, 32><<<dim3(up(fb.n[0], 32), up(fb.n[1], 16), zdim(fb.n[2])), 256, 0, st>>>(a);
-        else k_face_flux<1, 8, 32><<<dim3(up(fb.n[0], 32), up(fb.n[1], 8), zdim(fb.n[2])), 256, 0, st>>>(a);
+        if (tall) launch_after(k_face_flux<1, 16, 32>, dim3(up(fb.n[0], 32), up(fb.n[1], 16), zdim(fb.n[2])), 256, 0, st, a);
+        else launch_after(k_face_flux<1, 8, 32>, dim3(up(fb.n[0], 32), up(fb.n[1], 8), zdim(fb.n[2])), 256, 0, st, a);
     } else {
-        if (tall) k_face_flux<2, 16, 32><<<dim3(up(fb.n[0], 32), up(fb.n[2], 16), zdim(fb.n[1])), 256, 0, st>>>(a);
-        else k_face_flux<2, 8, 32><<<dim3(up(fb.n[0], 32), up(fb.n[2], 8), zdim(fb.n[1])), 256, 0, st>>>(a);
+        if (tall) launch_after(k_face_flux<2, 16, 32>, dim3(up(fb.n[0], 32), up(fb.n[2], 16), zdim(fb.n[1])), 256, 0, st, a);
+        else launch_after(k_face_flux<2, 8, 32>, dim3(up(fb.n[0], 32), up(fb.n[2], 8), zdim(fb.n[1])), 256, 0, st, a);
     }
     return cudaGetLastError();
 }
@@ -371,6 +372,7 @@ cudaError_t launch_face_flux(const BoxIdx& fb, int dir, int specid, const A4& ph
 __global__ void __launch_bounds__(128) k_dsdt(BoxIdx b, int dim, int specid, A4 f0, A4 f1, A4 f2, A4 rxn, A4 dsdt,
                                               double dx0, double dx1, double dx2)
 {
+    grid_wait();
     const int ii = blockIdx.x * 128 + threadIdx.x;
     if (ii >= b.n[0]) return;
     const int i = b.lo[0] + ii;
@@ -390,7 +392,7 @@ cudaError_t launch_dsdt(const BoxIdx& b, int dim, int specid, const A4 flux[3], 
     ProfScope ps("k_dsdt", st);
     const int64_t rows = (int64_t)b.n[1] * b.n[2];
     const dim3 g((unsigned)((b.n[0] + 127) / 128), (unsigned)(rows < 65535 ? rows : 65535));
-    k_dsdt<<<g, 128, 0, st>>>(b, dim, specid, flux[0], flux[1], flux[2], rxn, dsdt, dx[0], dx[1], dx[2]);
+    launch_after(k_dsdt, g, 128, 0, st, b, dim, specid, flux[0], flux[1], flux[2], rxn, dsdt, dx[0], dx[1], dx[2]);
     return cudaGetLastError();
 }
 
@@ -400,6 +402,7 @@ cudaError_t launch_dsdt(const BoxIdx& b, int dim, int specid, const A4 flux[3], 
 template <int DIM>
 __global__ void __launch_bounds__(kJouleThreads) k_joule(const __grid_constant__ TransportArgs a, int64_t ntiles)
 {
+    grid_wait();
     using JT = JouleTile<DIM>;
     constexpr int E0 = JT::X + 2, E1 = JT::Y + 2 * (DIM > 1), E2 = JT::Z + 2 * (DIM > 2);
     __shared__ double sN[E0 * E1 * E2];
@@ -458,9 +461,9 @@ cudaError_t launch_joule(const BoxIdx& b, int dim, const A4& sb, const A4& rxn, 
                                   : joule_tile_count<3>(a.lo, a.hi);
     const unsigned g = (unsigned)(nt < (1 << 30) ? nt : (1 << 30));
     ProfScope ps("k_joule", st);
-    if (dim == 1) k_joule<1><<<g, kJouleThreads, 0, st>>>(a, nt);
-    else if (dim == 2) k_joule<2><<<g, kJouleThreads, 0, st>>>(a, nt);
-    else k_joule<3><<<g, kJouleThreads, 0, st>>>(a, nt);
+    if (dim == 1) launch_after(k_joule<1>, g, kJouleThreads, 0, st, a, nt);
+    else if (dim == 2) launch_after(k_joule<2>, g, kJouleThreads, 0, st, a, nt);
+    else launch_after(k_joule<3>, g, kJouleThreads, 0, st, a, nt);
     return cudaGetLastError();
 }
 
@@ -803,7 +806,7 @@ static cudaError_t launch_tr(const TransportArgs& a, cudaStream_t st)
     }
     unsigned nt = (unsigned)a.ntile[0] * a.ntile[1] * a.ntile[2];
     ProfScope ps("k_transport", st);
-    k_transport<DIM, PREC, MINB><<<nt, TS::NTH, smem, st>>>(a);
+    launch_after(k_transport<DIM, PREC, MINB>, nt, TS::NTH, smem, st, a);
     return cudaGetLastError();
 }
 
@@ -879,6 +882,7 @@ static cudaError_t launch_tr_v(const TransportArgs& a, cudaStream_t st)
 template <int DIM, int PREC>
 __global__ void __launch_bounds__(kJouleThreads, 3) k_joule_pre(const __grid_constant__ TransportArgs a, int64_t ntiles)
 {
+    grid_wait();
     __shared__ double sJ[DIM * joule_face_box<DIM>()];
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         joule_tile<DIM, PREC>(a, (int)t, sJ);
@@ -893,7 +897,7 @@ static cudaError_t launch_jp(const TransportArgs& a, cudaStream_t st)
     if (nt <= 0) return cudaSuccess;
     const unsigned g = (unsigned)(nt < (1 << 30) ? nt : (1 << 30));
     ProfScope ps("k_joule_pre", st);
-    k_joule_pre<DIM, PREC><<<g, kJouleThreads, 0, st>>>(a, nt);
+    launch_after(k_joule_pre<DIM, PREC>, g, kJouleThreads, 0, st, a, nt);
     return cudaGetLastError();
 }
 

@@ -15,6 +15,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "vd_kernels.cuh"
 
 namespace vd {
 
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(kMg2Threads) k_mg2d(const __grid_constant__ OP
                                                       typename OP::T* __restrict__ phi_out, double* corr,
                                                       unsigned long long* maxout)
 {
+    grid_wait();
     using T = typename OP::T;
     constexpr int W = kMg2W, R = kMg2R, H = kMg2H;
     __shared__ T sp[W * R], sr[W * R];

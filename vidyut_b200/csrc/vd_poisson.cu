@@ -130,6 +130,7 @@ __device__ __forceinline__ void stencil(const LevelT<T>& L, const BcInfo& bc, in
 template <int DIM>
 __global__ void __launch_bounds__(128) k_mg_rbgs(CLevel L, BcInfo bc, int color, int half, double* corr)
 {
+    grid_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     int ii[2], jj[2], kk[2];
     bool row[2], ok[2];
@@ -180,6 +181,7 @@ template <int DIM>
 __global__ void __launch_bounds__(128) k_mg_defect(Level P, BcInfo bc, CLevel E, double scale, int half,
                                                    double* blkmax)
 {
+    grid_wait();
     // two cells per thread, `half` apart along the slowest active direction (as in
     // k_mg_rbgs), with all their loads issued first
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -227,6 +229,7 @@ __global__ void __launch_bounds__(128) k_mg_defect(Level P, BcInfo bc, CLevel E,
 // P phi += the correction of the finest correction level
 __global__ void __launch_bounds__(128) k_mg_correct(Level P, CLevel E)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n[0]) return;
@@ -258,6 +261,7 @@ __device__ __forceinline__ float mg_restrict(const CLevel& F, const BcInfo& bc, 
 template <int DIM>
 __global__ void __launch_bounds__(128) k_mg_restrict(CLevel F, CLevel C, BcInfo bc)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C.n[0]) return;
@@ -315,6 +319,7 @@ __device__ __forceinline__ float mg_prolong(const CLevel& C, const BcInfo& bc, i
 template <int DIM>
 __global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo bc)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= F.n[0]) return;
@@ -339,6 +344,7 @@ struct MCoarse {
 template <int DIM>
 __global__ void __launch_bounds__(1024) k_mg_coarse(const __grid_constant__ MCoarse P, const __grid_constant__ BcInfo bc)
 {
+    grid_wait();
     extern __shared__ float smf[];
     __shared__ int soff[kCoarseMax + 1];  // where each level's arrays begin
     const int tid = threadIdx.x, nth = blockDim.x;
@@ -531,12 +537,12 @@ struct Mg {
         ProfScope ps("k_mg_rbgs", st);
         int half = 0;
         const dim3 g = grid_pairs(L, DIM, 2, &half);
-        k_mg_rbgs<DIM><<<g, 128, 0, st>>>(L, b, color, half, corr);
+        launch_after(k_mg_rbgs<DIM>, g, 128, 0, st, L, b, color, half, corr);
     }
     static void restrict_(const CLevel& F, const CLevel& C, const BcInfo& b, cudaStream_t st)
     {
         ProfScope ps("k_mg_restrict", st);
-        k_mg_restrict<DIM><<<grid_cells(C), 128, 0, st>>>(F, C, b);
+        launch_after(k_mg_restrict<DIM>, grid_cells(C), 128, 0, st, F, C, b);
     }
     static cudaError_t coarse(const MCoarse& P, const BcInfo& b, cudaStream_t st)
     {
@@ -548,13 +554,13 @@ struct Mg {
         const int64_t t = (int64_t)((P.lv[0].n[0] + 1) / 2) * P.lv[0].n[1] * P.lv[0].n[2];
         const unsigned nth = (unsigned)(t >= 1024 ? 1024 : (t + 31) / 32 * 32);
         ProfScope ps("k_mg_coarse", st);
-        k_mg_coarse<DIM><<<1, nth, 2 * cells * sizeof(float), st>>>(P, b);
+        launch_after(k_mg_coarse<DIM>, 1, nth, 2 * cells * sizeof(float), st, P, b);
         return cudaGetLastError();
     }
     static void prolong(const CLevel& F, const CLevel& C, const BcInfo& b, cudaStream_t st)
     {
         ProfScope ps("k_mg_prolong", st);
-        k_mg_prolong<DIM><<<grid_cells(F), 128, 0, st>>>(F, C, b);
+        launch_after(k_mg_prolong<DIM>, grid_cells(F), 128, 0, st, F, C, b);
     }
     static void defect(const Level& P, const BcInfo& b, const CLevel& E, double scale, double* blkmax,
                        cudaStream_t st)
@@ -562,7 +568,7 @@ struct Mg {
         ProfScope ps("k_mg_defect", st);
         int half = 0;
         const dim3 g = grid_pairs(P, DIM, 1, &half);
-        k_mg_defect<DIM><<<g, 128, 0, st>>>(P, b, E, scale, half, blkmax);
+        launch_after(k_mg_defect<DIM>, g, 128, 0, st, P, b, E, scale, half, blkmax);
     }
 };
 
@@ -583,6 +589,7 @@ MgOps mg_ops(int dim) { return dim == 1 ? mg_ops_of<1>() : dim == 2 ? mg_ops_of<
 
 __global__ void k_maxabs(const double* x, int64_t n, unsigned long long* out)
 {
+    grid_wait();
     double m = 0.0;
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < n; c += (int64_t)gridDim.x * blockDim.x)
         m = fmax(m, fabs(x[c]));
@@ -602,6 +609,7 @@ struct PoisArgs {
 // phi = the state's potential
 __global__ void k_pois_rhs(PoisArgs a, Level L)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < L.n[0]) {
@@ -624,6 +632,7 @@ struct D3 {
 
 __global__ void __launch_bounds__(128) k_pois_cell_fields(PoisArgs a, Level L, D3 dxs)
 {
+    grid_wait();
     const int ns = a.ns;
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -670,6 +679,7 @@ __global__ void __launch_bounds__(128) k_pois_cell_fields(PoisArgs a, Level L, D
 template <int D>
 __global__ void __launch_bounds__(128) k_pois_face_field(Level L, BcInfo bc, A4 ef, double dx)
 {
+    grid_wait();
     const int j = blockIdx.y, k = blockIdx.z;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nf0 = L.n[0] + (D == 0);
@@ -864,7 +874,7 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
 
     {
         ProfScope ps("k_pois_rhs", st);
-        k_pois_rhs<<<grid_cells(P), 128, 0, st>>>(pa, P);
+        launch_after(k_pois_rhs, grid_cells(P), 128, 0, st, pa, P);
     }
     if ((rc = launch_check("k_pois_rhs"))) return rc;
     double rhs_scale = 0.0;
@@ -904,8 +914,8 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         op.bc = bc0;
         ProfScope ps(up ? "k_mg_leg_up" : "k_mg_leg_down", st);
         const dim3 g = mg2d_grid(op.n);
-        if (up) k_mg2d<MOp2, true><<<g, kMg2Threads, 0, st>>>(op, lv[l].res, lv[l].phi, l == 0 ? P.phi : nullptr, nullptr);
-        else k_mg2d<MOp2, false><<<g, kMg2Threads, 0, st>>>(op, nullptr, lv[l].res, nullptr, nullptr);
+        if (up) launch_after(k_mg2d<MOp2, true>, g, kMg2Threads, 0, st, op, lv[l].res, lv[l].phi, l == 0 ? P.phi : nullptr, nullptr);
+        else launch_after(k_mg2d<MOp2, false>, g, kMg2Threads, 0, st, op, nullptr, lv[l].res, nullptr, nullptr);
     };
     auto vcycle = [&]() {
         for (int l = 0; l < lc; l++) {
@@ -935,7 +945,7 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         }
         if (!fine) {  // the whole cycle was one launch, or the bottom solve
             ProfScope ps("k_mg_correct", st);
-            k_mg_correct<<<grid_cells(P), 128, 0, st>>>(P, lv[0]);
+            launch_after(k_mg_correct, grid_cells(P), 128, 0, st, P, lv[0]);
         }
     };
     // the max of the n doubles (non-negative doubles order like their bit patterns)
@@ -943,7 +953,7 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
         cudaMemsetAsync(d_max, 0, sizeof(unsigned long long), st);
         {
             ProfScope ps("k_maxabs", st);
-            k_maxabs<<<grid_of(nx), 256, 0, st>>>(x, nx, d_max);
+            launch_after(k_maxabs, grid_of(nx), 256, 0, st, x, nx, d_max);
         }
         unsigned long long h = 0;
         cudaError_t ce = cudaMemcpyAsync(&h, d_max, sizeof(h), cudaMemcpyDeviceToHost, st);
@@ -985,7 +995,7 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
     D3 dxs{{prm->dx[0], prm->dx[1], prm->dx[2]}};
     {
         ProfScope ps("k_pois_cell_fields", st);
-        k_pois_cell_fields<<<grid_cells(P), 128, 0, st>>>(pa, P, dxs);
+        launch_after(k_pois_cell_fields, grid_cells(P), 128, 0, st, pa, P, dxs);
     }
     if (!prm->cs_technique)
         for (int d = 0; d < dim; d++) {
@@ -995,9 +1005,9 @@ extern "C" int vd_poisson_solve(const vd_box* bx, vd_array4 state, const vd_arra
             ProfScope ps("k_pois_face_field", st);
             const dim3 g((unsigned)((nf[0] + 127) / 128), (unsigned)nf[1], (unsigned)nf[2]);
             const A4 efd(efield_ec[d]);
-            if (d == 0) k_pois_face_field<0><<<g, 128, 0, st>>>(P, bc, efd, prm->dx[0]);
-            else if (d == 1) k_pois_face_field<1><<<g, 128, 0, st>>>(P, bc, efd, prm->dx[1]);
-            else k_pois_face_field<2><<<g, 128, 0, st>>>(P, bc, efd, prm->dx[2]);
+            if (d == 0) launch_after(k_pois_face_field<0>, g, 128, 0, st, P, bc, efd, prm->dx[0]);
+            else if (d == 1) launch_after(k_pois_face_field<1>, g, 128, 0, st, P, bc, efd, prm->dx[1]);
+            else launch_after(k_pois_face_field<2>, g, 128, 0, st, P, bc, efd, prm->dx[2]);
         }
     if ((rc = launch_check("potential fields"))) return rc;
     // ghosts of the potential, the cell field and the reduced field

@@ -1187,6 +1187,7 @@ const int j = GRP == 1 ? 0 : q / RG::NRUN, r = q - j * RG::NRUN;
 template <int DIM, int PREC, int MINB>
 __global__ void __launch_bounds__(default_nth<DIM, PREC>(), MINB) k_transport(const __grid_constant__ TransportArgs a)
 {
+    grid_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using TS = typename DefaultTile<DIM, PREC>::T;
     transport_tile_update<DIM, PREC, TS, group_fit<DIM, PREC, TS, MINB>()>(a, blockIdx.x, smem_raw);
