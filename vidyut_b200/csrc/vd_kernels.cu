@@ -1019,17 +1019,25 @@ __global__ void __launch_bounds__(256) k_time_scales(BoxIdx b, int dim, A4 st, T
         }
         const double emag = sqrt(esum);
         double nd = 0.0;
-        for (int s = 0; s < ns; s++) nd += st.p[o + (int64_t)s * st.ns];
+#pragma unroll 8
+        for (int s = 0; s < ns; s++) nd += __ldg(st.p + o + (int64_t)s * st.ns);
         const double dc = a.const_ele_trans ? a.ele_diff / nd : diff_fp64(eidx, etemp, nd, a.Tg, emag);
         const double mu = a.const_ele_trans ? a.ele_mob / nd : mob_fp64(eidx, etemp, nd, a.Tg, emag);
         m[0] = fmax(m[0], fabs(mu) * emag);
         m[1] = fmax(m[1], dc);
         m[2] = fmax(m[2], fabs(mu) * st.p[o + (int64_t)eidx * st.ns]);
     }
+    __shared__ double wm[3][8];
     for (int q = 0; q < 3; q++) {
         double v = m[q];
         for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, off));
-        if ((threadIdx.x & 31) == 0) atomicMax(out + q, (unsigned long long)__double_as_longlong(v));
+        if ((threadIdx.x & 31) == 0) wm[q][threadIdx.x >> 5] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double v = wm[threadIdx.x][0];
+        for (int w = 1; w < 8; w++) v = fmax(v, wm[threadIdx.x][w]);
+        atomicMax(out + threadIdx.x, (unsigned long long)__double_as_longlong(v));
     }
 }
 

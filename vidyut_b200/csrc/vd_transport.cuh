@@ -228,19 +228,25 @@ __device__ __forceinline__ double joule_face(const TransportArgs& a, int D, cons
     const double nel = p[ol + eidx * cs], ner = p[orr + eidx * cs];
     const double ne = 0.5 * (nel + ner);
     const double ef = a.cs_technique ? evf_d : a.ef[D](g[0], g[1], g[2]);
-    const double gn = a.gradne_from_state ? (ner - nel) / a.dx[D] : a.gne[D](g[0], g[1], g[2]);
+    const double gn = a.gradne_from_state ? (ner - nel) * a.idx[D] : a.gne[D](g[0], g[1], g[2]);
     const double ndens = 0.5 * (a.Nv.p[a.Nv.off(l[0], l[1], l[2])] + a.Nv.p[a.Nv.off(g[0], g[1], g[2])]);
     double emag = 0.0;
     if (c_mech.emag_e) emag = face_emag(a, ol, orr, dim);
     double mu, dc;
     if (a.const_ele_trans) {
-        mu = a.ele_mob / ndens;
-        dc = a.ele_diff / ndens;
+        const double rn = rcp64(ndens);
+        mu = a.ele_mob * rn;
+        dc = a.ele_diff * rn;
     } else {
-        mu = mob_fp64(eidx, etemp, ndens, a.Tg, emag);
+        // the usual electron models without a division: two of them and a square root
+        // per face were a fifth of the pass (128^3 0.218 -> 0.182 ms)
+        if (c_mech.mob_kind[eidx] == VD_MOB_ELECTRON)
+            mu = c_mech.mob_c[eidx] * rsqrt(etemp) * rcp64(ndens * c_mech.mob_p0[eidx]);
+        else
+            mu = mob_fp64(eidx, etemp, ndens, a.Tg, emag);
         // the usual electron diffusion model refers to the electron mobility itself
         if (c_mech.diff_kind[eidx] == VD_DIFF_TE_ABSMOB && c_mech.diff_ref[eidx] == eidx)
-            dc = c_mech.diff_factor[eidx] * (etemp / EV) * fabs(mu);
+            dc = c_mech.diff_factor[eidx] * (etemp * (1.0 / EV)) * fabs(mu);
         else
             dc = diff_fp64(eidx, etemp, ndens, a.Tg, emag);
     }
