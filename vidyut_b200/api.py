@@ -15,6 +15,7 @@ status and message; nothing falls back to the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from dataclasses import dataclass
 
 import numpy as np
@@ -51,12 +52,27 @@ _I3, _D3 = C.c_int32 * 3, C.c_double * 3
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-def _i3(v):
+# Small constant arguments (boundary codes, cell counts, spacings, boxes) by value: the
+# library only reads them.
+@functools.lru_cache(maxsize=256)
+def _i3_of(v):
     return _I3(*map(int, v))
 
 
-def _d3(v):
+@functools.lru_cache(maxsize=256)
+def _d3_of(v):
     return _D3(*map(float, v))
+
+
+_box_of = functools.lru_cache(maxsize=256)(abi.make_box)
+
+
+def _i3(v):
+    return _i3_of(v if type(v) is tuple else tuple(v))
+
+
+def _d3(v):
+    return _d3_of(v if type(v) is tuple else tuple(v))
 
 
 def _a4_bytes(t: torch.Tensor, begin) -> bytes:
@@ -121,7 +137,7 @@ def compute_explicit_flux(dc: DeviceCase, d: int, specid: int, fx: torch.Tensor,
                           vel_species=0, stream=None) -> None:
     L = abi.lib()
     c = dc.case
-    rc = L.vd_compute_explicit_flux(dc.box(), d, specid, dc.sb(), _i3(bclo), _i3(bchi), _I3(), _i3(c.hi),
+    rc = L.vd_compute_explicit_flux(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), d, specid, dc.sb(), _i3(bclo), _i3(bchi), _I3(), _i3(c.hi),
                                     t_a4(fx, _ORIGIN), Tg, 0.0, 0.0, _d3(c.dx), dt, hyp_order, udv, weno,
                                     _d3(uvel), vel_species, _stream(stream))
     abi.check(rc, "vd_compute_explicit_flux")
@@ -132,21 +148,21 @@ def compute_dsdt(dc: DeviceCase, specid: int, flux: list, rxn: torch.Tensor, dsd
     L = abi.lib()
     fb = [_a4_bytes(f, _ORIGIN) for f in flux]
     fl = abi.A4x3.from_buffer_copy(b"".join(fb[d] if d < len(fb) else fb[0] for d in range(3)))
-    rc = L.vd_compute_dsdt(dc.box(), specid, fl, t_a4(rxn, _ORIGIN), t_a4(dsdt, _ORIGIN), _d3(dc.case.dx),
+    rc = L.vd_compute_dsdt(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), specid, fl, t_a4(rxn, _ORIGIN), t_a4(dsdt, _ORIGIN), _d3(dc.case.dx),
                            _stream(stream))
     abi.check(rc, "vd_compute_dsdt")
 
 
 def reaction_source(dc: DeviceCase, rxn: torch.Tensor, Tg=300.0, stream=None) -> None:
     L = abi.lib()
-    rc = L.vd_reaction_source(dc.box(), dc.sb(), t_a4(rxn, (0, 0, 0)), Tg, 0.0, 0.0, _stream(stream))
+    rc = L.vd_reaction_source(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), t_a4(rxn, (0, 0, 0)), Tg, 0.0, 0.0, _stream(stream))
     abi.check(rc, "vd_reaction_source")
 
 
 def compute_elecenergy_source(dc: DeviceCase, rxn: torch.Tensor, dsdt_energy: torch.Tensor,
                               phi_new: torch.Tensor, prm: abi.VdParams, stream=None) -> None:
     L = abi.lib()
-    rc = L.vd_elecenergy_source(dc.box(), dc.sb(), t_a4(rxn, (0, 0, 0)), dc.face_a4s("efield"),
+    rc = L.vd_elecenergy_source(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), t_a4(rxn, (0, 0, 0)), dc.face_a4s("efield"),
                                 dc.face_a4s("gradne"), t_a4(dsdt_energy, (0, 0, 0)), t_a4(phi_new, (0, 0, 0)),
                                 C.byref(prm), _stream(stream))
     abi.check(rc, "vd_elecenergy_source")
@@ -155,7 +171,7 @@ def compute_elecenergy_source(dc: DeviceCase, rxn: torch.Tensor, dsdt_energy: to
 def explicit_update_all(dc: DeviceCase, prm: abi.VdParams, phi_new: torch.Tensor, dsdt: torch.Tensor | None = None,
                         rxn: torch.Tensor | None = None, stream=None) -> None:
     L = abi.lib()
-    rc = L.vd_explicit_update_all(dc.box(), dc.sb(), dc.face_a4s("efield"), dc.face_a4s("gradne"),
+    rc = L.vd_explicit_update_all(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), dc.face_a4s("efield"), dc.face_a4s("gradne"),
                                   t_a4(phi_new, (0, 0, 0)),
                                   t_a4(dsdt, (0, 0, 0)) if dsdt is not None else abi.null_array4(),
                                   t_a4(rxn, (0, 0, 0)) if rxn is not None else abi.null_array4(),
@@ -166,7 +182,7 @@ def explicit_update_all(dc: DeviceCase, prm: abi.VdParams, phi_new: torch.Tensor
 def box_checksums(dc: DeviceCase, rxn: torch.Tensor, phi_new: torch.Tensor, stream=None) -> np.ndarray:
     L = abi.lib()
     out = torch.zeros(4, dtype=torch.float64, device=rxn.device)
-    rc = L.vd_box_checksums(dc.box(), t_a4(rxn, (0, 0, 0)), t_a4(phi_new, (0, 0, 0)), out.data_ptr(),
+    rc = L.vd_box_checksums(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), t_a4(rxn, (0, 0, 0)), t_a4(phi_new, (0, 0, 0)), out.data_ptr(),
                             _stream(stream))
     abi.check(rc, "vd_box_checksums")
     return out.cpu().numpy()
@@ -180,7 +196,7 @@ def explicit_update_all_noalloc(dc: DeviceCase, prm: abi.VdParams, phi_new: torc
     GPU): its scratch comes from a fixed VD_NOALLOC_SCRATCH_BYTES array in the
     library.  Boxes whose scratch would not fit raise VidyutError(ERR_NOMEM)."""
     L = abi.lib()
-    rc = L.vd_explicit_update_all_noalloc(dc.box(), dc.sb(), dc.face_a4s("efield"),
+    rc = L.vd_explicit_update_all_noalloc(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), dc.face_a4s("efield"),
                                           dc.face_a4s("gradne"), t_a4(phi_new, (0, 0, 0)),
                                           t_a4(dsdt, (0, 0, 0)) if dsdt is not None else abi.null_array4(),
                                           t_a4(rxn, (0, 0, 0)) if rxn is not None else abi.null_array4(),
@@ -435,7 +451,7 @@ def poisson_solve(dc: DeviceCase, prm: abi.VdParams, pp: abi.VdPoissonParams, st
     st = state if state is not None else dc.state
     nv = C.c_int32()
     rr = C.c_double()
-    rc = abi.lib().vd_poisson_solve(dc.box(), t_a4(st, dc.case.state_begin()), dc.face_a4s("efield"),
+    rc = abi.lib().vd_poisson_solve(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), t_a4(st, dc.case.state_begin()), dc.face_a4s("efield"),
                                     C.byref(prm), C.byref(pp), C.byref(nv), C.byref(rr), _stream(stream))
     abi.check(rc, "vd_poisson_solve")
     return nv.value, rr.value
@@ -468,7 +484,7 @@ def implicit_species_solve(dc: DeviceCase, spec: int, state_old: torch.Tensor, d
     g = None
     if gradne is not None:
         g = (abi.VdArray4 * 3)(*[t_a4(gradne[d], (0, 0, 0)) for d in range(3)])
-    rc = abi.lib().vd_implicit_species_solve(dc.box(), dc.sb(), t_a4(state_old, dc.case.state_begin()),
+    rc = abi.lib().vd_implicit_species_solve(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), t_a4(state_old, dc.case.state_begin()),
                                              t_a4(dsdt, (0, 0, 0)), t_a4(phi_new, (0, 0, 0)), g, C.byref(prm),
                                              C.byref(dp), C.byref(nv), C.byref(rr), _stream(stream))
     abi.check(rc, "vd_implicit_species_solve")
@@ -541,6 +557,6 @@ def time_scales(dc: DeviceCase, prm: abi.VdParams, stream=None):
     """(dt_edrift, dt_ediff, dt_diel_relax) of the case's current state
     (Vidyut::find_time_scales)."""
     out = (C.c_double * 3)()
-    abi.check(abi.lib().vd_time_scales(dc.box(), dc.sb(), C.byref(prm), out, _stream(stream)),
+    abi.check(abi.lib().vd_time_scales(_box_of(dc.case.lo, dc.case.hi, dc.case.dim), dc.sb(), C.byref(prm), out, _stream(stream)),
               "vd_time_scales")
     return tuple(out)
