@@ -216,7 +216,8 @@ int spec_compile_only(const VdMechDev& m, size_t* cubin_bytes);
 // Grids of many waves gain nothing from it (3-D FP64 step of 128^3 2.86 ms without,
 // 2.89 ms with); small ones do: 1-D 300 cells 30.7 -> 27.9 us, 467 x 509 mixed 112 ->
 // 104 us, electron solve of 512^2 787 -> 753 us, per-call 64^3 step 772 -> 676 us.
-inline int overlap_grid(dim3 g) { return (int64_t)g.x * g.y * g.z <= 20 * 148; }
+constexpr int kOverlapCtas = 20 * 148;
+inline int overlap_grid(dim3 g) { return (int64_t)g.x * g.y * g.z <= kOverlapCtas; }
 template <class... P, class... A>
 inline cudaError_t launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                 const A&... args)
@@ -240,8 +241,11 @@ inline cudaError_t launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t s
         held);
 }
 #ifdef __CUDACC__
+// (large grids are not launched so, and skip the two instructions: in each of 131,072
+// CTAs of one cell per thread they cost more than the work saved, 32 -> 45 us)
 __device__ __forceinline__ void grid_wait()
 {
+    if ((long long)gridDim.x * gridDim.y * gridDim.z > kOverlapCtas) return;
     asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
 }
 #endif

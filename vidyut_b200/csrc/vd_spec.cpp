@@ -205,7 +205,7 @@ std::string gen_prep_kernel(const VdMechDev& m, int prec, bool source = false)
     // of (box, chunk of kPrepChunk cells)), both around one per-cell function
     o << "__device__ __forceinline__ void vd_spec_cell_" << sfx << "(const PrepArgs& a, i64 idx);\n";
     o << "extern \"C\" __global__ void " << lb << " vd_spec_prep_" << sfx << "(const PrepArgs a)\n{\n"
-      << "  asm volatile(\"griddepcontrol.launch_dependents;\\n\\tgriddepcontrol.wait;\" ::: \"memory\");\n"
+      << "  if (gridDim.x <= " << kOverlapCtas << ")\n    asm volatile(\"griddepcontrol.launch_dependents;\\n\\tgriddepcontrol.wait;\" ::: \"memory\");\n"
       << "  const i64 ntot = (i64)(a.ghi[0] - a.glo[0] + 1) * (a.ghi[1] - a.glo[1] + 1) * (a.ghi[2] - a.glo[2] + 1);\n"
       << "  for (i64 idx = blockIdx.x * (i64)blockDim.x + threadIdx.x; idx < ntot; idx += (i64)gridDim.x * blockDim.x)\n"
       << "    vd_spec_cell_" << sfx << "(a, idx);\n}\n";
