@@ -618,9 +618,20 @@ __device__ __forceinline__ void ghost_cell(const GhostArgs& a, int64_t idx)
         src[d] = a.periodic[d] ? a.lo[d] + ((g - 1) % n[d]) : a.hi[d];
     }
     const int64_t od = a.st.off(dst[0], dst[1], dst[2]), os = a.st.off(src[0], src[1], src[2]);
-    for (int q = 0; q < a.ncomp; q++) {
-        const int64_t co = (int64_t)a.comps[q] * a.st.ns;
-        a.st.p[od + co] = a.st.p[os + co];
+    // several components' loads in flight before their stores (one by one, each load
+    // waited for the store before it; the source is never a ghost cell)
+    constexpr int CH = 5;
+    for (int q0 = 0; q0 < a.ncomp; q0 += CH) {
+        double v[CH];
+        int64_t co[CH];
+#pragma unroll
+        for (int k = 0; k < CH; k++) {
+            co[k] = (int64_t)a.comps[q0 + k < a.ncomp ? q0 + k : a.ncomp - 1] * a.st.ns;
+            v[k] = a.st.p[os + co[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < CH; k++)
+            if (q0 + k < a.ncomp) a.st.p[od + co[k]] = v[k];
     }
 }
 

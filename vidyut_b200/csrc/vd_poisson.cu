@@ -374,6 +374,62 @@ __global__ void __launch_bounds__(128) k_mg_prolong(CLevel F, CLevel C, BcInfo b
     F.phi[lin(F, i, j, k)] += mg_prolong<DIM>(C, bc, i, j, k);
 }
 
+// The same prolongation in 3-D for four consecutive fine cells per thread (rows of whole
+// 16-byte groups): the four rows of coarse cells are read once for them, and the fine
+// row in one access.  All prolongations of a 256^3 solve (11 cycles) 1.45 -> 0.65 ms.
+__global__ void __launch_bounds__(128) k_mg_prolong4(CLevel F, CLevel C, BcInfo bc)
+{
+    grid_wait();
+    const int i0 = 4 * (blockIdx.x * 32 + threadIdx.x % 32);
+    const int j = blockIdx.y * 4 + threadIdx.x / 32, k = blockIdx.z;
+    if (i0 >= F.n[0] || j >= F.n[1]) return;
+    // along y and z: the two coarse rows and their weights, as mg_prolong has them
+    const int f[3] = {i0, j, k};
+    const int str[3] = {1, C.n[0], C.n[0] * C.n[1]};
+    int off[3][2];
+    float w[3][2];
+#pragma unroll
+    for (int d = 1; d < 3; d++) {
+        const int ci = f[d] >> 1, q = ci + ((f[d] & 1) ? 1 : -1);
+        off[d][0] = ci * str[d];
+        w[d][0] = 0.75f;
+        if (q < 0) {
+            off[d][1] = off[d][0];
+            w[d][1] = bc.dir_lo[d] ? -0.25f : 0.25f;
+        } else if (q >= C.n[d]) {
+            off[d][1] = off[d][0];
+            w[d][1] = bc.dir_hi[d] ? -0.25f : 0.25f;
+        } else {
+            off[d][1] = q * str[d];
+            w[d][1] = 0.25f;
+        }
+    }
+    // along x: coarse cells c0 - 1 .. c0 + 2 (beyond a domain face the parent itself)
+    const int c0 = i0 >> 1, cn = C.n[0];
+    const bool lo = c0 > 0, hi = c0 + 2 < cn;
+    const float wl = lo || !bc.dir_lo[0] ? 0.25f : -0.25f, wh = hi || !bc.dir_hi[0] ? 0.25f : -0.25f;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int mz = 0; mz < 2; mz++)
+#pragma unroll
+        for (int my = 0; my < 2; my++) {
+            const float* r = C.phi + (off[1][my] + off[2][mz]) + c0;
+            const float a = r[0], b = r[1], l = lo ? r[-1] : a, h = hi ? r[2] : b;
+            const float ww = w[1][my] * w[2][mz];
+            acc[0] += ww * (0.75f * a + wl * l);
+            acc[1] += ww * (0.75f * a + 0.25f * b);
+            acc[2] += ww * (0.75f * b + 0.25f * a);
+            acc[3] += ww * (0.75f * b + wh * h);
+        }
+    float4* p = reinterpret_cast<float4*>(F.phi + lin(F, i0, j, k));
+    float4 v = *p;
+    v.x += acc[0];
+    v.y += acc[1];
+    v.z += acc[2];
+    v.w += acc[3];
+    *p = v;
+}
+
 // The coarse end of the V-cycle in one CTA: every level from the first whose arrays
 // fit shared memory (about 128^2 or 27^3 cells) down to the coarsest grid and back,
 // with a barrier between half sweeps: one launch instead of eleven per level and a
@@ -613,6 +669,10 @@ struct Mg {
     static void prolong(const CLevel& F, const CLevel& C, const BcInfo& b, cudaStream_t st)
     {
         ProfScope ps("k_mg_prolong", st);
+        if (DIM == 3 && F.n[0] % 4 == 0 && (uintptr_t)F.phi % 16 == 0) {
+            launch_after(k_mg_prolong4, dim3((F.n[0] + 127) / 128, (F.n[1] + 3) / 4, F.n[2]), 128, 0, st, F, C, b);
+            return;
+        }
         launch_after(k_mg_prolong<DIM>, grid_cells(F), 128, 0, st, F, C, b);
     }
     static void defect(const Level& P, const BcInfo& b, const CLevel& E, double scale, double* blkmax,
