@@ -528,7 +528,7 @@ int spec_compile_only(const VdMechDev& m, size_t* cubin_bytes)
         nvrtcDestroyProgram(&prog);
         return 3;
     }
-    g_spec_err = log.substr(0, 2000);  // resource usage reported by ptxas
+    g_spec_err = log.substr(0, 4000);  // resource usage reported by ptxas
     nvrtcGetCUBINSize(prog, cubin_bytes);
     nvrtcDestroyProgram(&prog);
     return 0;
